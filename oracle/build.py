@@ -116,7 +116,7 @@ def _write_forwarders(ref: str, inc_dir: str) -> None:
 def build_ref(ref: str = REF_DEFAULT, force: bool = False) -> str | None:
     """Compile the reference Cores + shims + driver.  Returns the .so path, or
     None when the reference tree is absent (then any earlier build is kept)."""
-    if not os.path.isdir(ref):
+    if not os.path.isfile(os.path.join(ref, REF_SOURCES[0])):   # no tree, or an empty folder in its place
         return REF_SO if os.path.exists(REF_SO) else None
     shim_dir = os.path.join(HERE, "ref_shims")
     deps = [os.path.join(ref, s) for s in REF_SOURCES] + [
@@ -162,7 +162,7 @@ def build_ref_gpu(ref: str = REF_DEFAULT, force: bool = False) -> str | None:
     shims + the driver into baseline/_ref/libbpcuda_ref.so.  Returns the .so
     path, or None when the reference tree is absent (an earlier build is
     kept)."""
-    if not os.path.isdir(ref):
+    if not os.path.isfile(os.path.join(ref, GPU_CU[0])):
         return GPU_SO if os.path.exists(GPU_SO) else None
     shim = os.path.join(HERE, "ref_shims", "ipp_mkl_shims.cpp")
     drv = os.path.join(HERE, "ref_gpu", "bpcuda_driver.cpp")
