@@ -13,6 +13,7 @@ import argparse
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
@@ -57,7 +58,7 @@ def _run(cmd, verbose):
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     hdr_time = max(os.path.getmtime(h) for h in headers())
-    objs, relink = [], force or not os.path.exists(LIB)
+    objs, relink, jobs = [], force or not os.path.exists(LIB), []
     for src in sources():
         obj = os.path.join(OBJ, os.path.basename(src) + ".o")
         objs.append(obj)
@@ -65,7 +66,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
                 and os.path.getmtime(obj) >= hdr_time):
             continue
         flags = CU_FLAGS if src.endswith(".cu") else COMMON
-        _run([NVCC] + flags + ["-c", src, "-o", obj], verbose)
+        jobs.append([NVCC] + flags + ["-c", src, "-o", obj])
+    if jobs:   # side by side: the backprojection's instances take minutes one after another
+        with ThreadPoolExecutor(min(len(jobs), os.cpu_count() or 1)) as pool:
+            list(pool.map(lambda cmd: _run(cmd, verbose), jobs))
         relink = True
     if relink or any(os.path.getmtime(o) > os.path.getmtime(LIB) for o in objs):
         _run([NVCC, "-shared"] + ARCH + ["-o", LIB] + objs, verbose)

@@ -67,10 +67,10 @@ __global__ void __launch_bounds__(256) bp_adjoint_kernel(AdjParams p) {
     for (int n = 0; n < p.nv; ++n, P4 += 3, qb += p.q_frame) {
         const float4 r0 = __ldg(P4), r1 = __ldg(P4 + 1), r2 = __ldg(P4 + 2);
         const XYTerms xy = bp_xy_terms(ax, ay, r0, r1, r2);
-        const float rxy = WZ ? 0.0f : rcp_rn_nr(xy.W);
+        const Recip rc = WZ ? Recip{0.0f, 0.0f} : bp_recip(xy.W);
 #pragma unroll
         for (int k = 0; k < ZPT; ++k) {
-            const float2 uv = bp_uv(xy, bp_w_r<WZ>(xy, rxy, az[k], r2.z), az[k], r0.z, r1.z);
+            const float2 uv = bp_uv<false, WZ>(xy, rc, az[k], r0.z, r1.z, r2.z);
             const bool in = (uv.x >= 0.0f) & (uv.x <= umax) & (uv.y >= 0.0f) & (uv.y <= vmax);
             if (in && rt[k] != 0.0f) {
                 // floor by the 2^23 add rounded toward -inf (exact for 0 <= u, v < 2^23)
@@ -142,13 +142,13 @@ __global__ void __launch_bounds__(256) geometry_gradient_kernel(AdjParams p) {
         if (valid) {
             const float4 r0 = __ldg(P4), r1 = __ldg(P4 + 1), r2 = __ldg(P4 + 2);
             const XYTerms xy = bp_xy_terms(ax, ay, r0, r1, r2);
-            const float rxy = WZ ? 0.0f : rcp_rn_nr(xy.W);
+            const Recip rc = WZ ? Recip{0.0f, 0.0f} : bp_recip(xy.W);
             const float4* __restrict__ q = p.q4 + (size_t)n * p.q_frame;
             const float2* __restrict__ tw = p.tw + (size_t)((p.v0 + n) % p.num_views) * p.U;
 #pragma unroll
             for (int k = 0; k < ZPT; ++k) {
-                const float2 wr = bp_w_r<WZ>(xy, rxy, az[k], r2.z);
-                const float2 uv = bp_uv(xy, wr, az[k], r0.z, r1.z);
+                const float2 wr = bp_w_r<WZ>(xy, rc, az[k], r2.z);
+                const float2 uv = bp_uv<false, WZ>(xy, rc, az[k], r0.z, r1.z, r2.z);
                 const bool in = (uv.x >= 0.0f) & (uv.x <= umax) & (uv.y >= 0.0f) & (uv.y <= vmax);
                 if (in && rt[k] != 0.0f) {
                     const float2 t = padd_rm(uv, f2(kMagic, kMagic));          // 2^23 + floor

@@ -79,9 +79,8 @@ constexpr int kMagicBits = 0x4B000000;  // bit pattern of 2^23
 
 // Sample point of the FP32 form, as BPCore rounds it (BPCore.cpp:120-145,
 // 207-220): Uxy = x*P0 + (y*P1 + P3), likewise V, W; U = Uxy + z*P2 etc.,
-// every product and sum rounded separately; u = RN(U / W) + 0.5 from one
-// correctly rounded reciprocal r = RN(1/W) and Markstein's correction
-// q = RN(q0 + RN(U - W q0) r), q0 = RN(U r).
+// every product and sum rounded separately; u = RN(U / W) + 0.5
+// (bp_quotient2).
 struct XYTerms { float U, V, W; };
 
 __device__ __forceinline__ XYTerms bp_xy_terms(float ax, float ay, const float4& r0, const float4& r1,
@@ -104,22 +103,63 @@ __device__ __forceinline__ float rcp_rn_nr(float w) {
     return fmaf(fmaf(-w, y, 1.0f), y, y);
 }
 
-// W and r = RN(1/W) at slice coordinate az (W independent of z unless WZ).
+// 1/W as a float r = RN(1/W) and the float nearest to what r lacks, rl =
+// RN(RN(1 - W r) r): the residual 1 - W r is exact, so r + rl is 1/W to 2^-47.
+struct Recip { float r, rl; };
+
+__device__ __forceinline__ Recip bp_recip(float W) {
+    const float r = rcp_rn_nr(W);
+    return {r, __fmul_rn(fmaf(-W, r, 1.0f), r)};
+}
+
+// U / W of both lanes.  EXACT: correctly rounded, from r and Markstein's
+// correction q = RN(q0 + RN(U - W q0) r), q0 = RN(U r).  Otherwise
+// RN(U r + RN(U rl)), one operation less (5 % of the FP32 loop): the sum is within 2^-47 of U / W
+// before its one rounding, so it is the correctly rounded quotient but where
+// U / W lies that close to the middle between two floats (none of 1.6e8 random
+// quotients), and then the other of the two, off by half a unit in the last
+// place like the one it stands for.
+template <bool EXACT>
+__device__ __forceinline__ float2 bp_quotient2(float2 U, float W, const Recip& rc) {
+    const float2 rr = f2(rc.r, rc.r);
+    if constexpr (EXACT) {
+        const float2 q0 = pmul(U, rr);
+        const float2 rem = pfma(f2(-W, -W), q0, U);           // exact remainder
+        return pfma(rem, rr, q0);
+    }
+    return pfma(U, rr, pmul(U, f2(rc.rl, rc.rl)));
+}
+
+template <bool EXACT>
+__device__ __forceinline__ float bp_quotient(float U, float W, const Recip& rc) {
+    if constexpr (EXACT) {
+        const float q0 = __fmul_rn(U, rc.r);
+        return fmaf(fmaf(-W, q0, U), rc.r, q0);
+    }
+    return fmaf(U, rc.r, __fmul_rn(U, rc.rl));
+}
+
+// W and RN(1/W) at slice coordinate az (W independent of z unless WZ).
 template <bool WZ>
-__device__ __forceinline__ float2 bp_w_r(const XYTerms& t, float rxy, float az, float P10) {
+__device__ __forceinline__ float2 bp_w_r(const XYTerms& t, const Recip& rc, float az, float P10) {
     if (WZ) {
         const float W = __fadd_rn(t.W, __fmul_rn(az, P10));
         return f2(W, rcp_rn_nr(W));
     }
-    return f2(t.W, rxy);
+    return f2(t.W, rc.r);
 }
 
-__device__ __forceinline__ float2 bp_uv(const XYTerms& t, float2 wr, float az, float P2, float P6) {
+// (u, v) of the sample at slice coordinate az.  WZ: W and its reciprocal are
+// the slice's, and the quotient is Markstein's (rl would cost two operations
+// a sample to save one).
+template <bool EXACT, bool WZ>
+__device__ __forceinline__ float2 bp_uv(const XYTerms& t, const Recip& rc, float az, float P2, float P6, float P10) {
     const float2 UV = f2(__fadd_rn(t.U, __fmul_rn(az, P2)), __fadd_rn(t.V, __fmul_rn(az, P6)));
-    const float2 rr = f2(wr.y, wr.y);
-    const float2 q0 = pmul(UV, rr);
-    const float2 rem = pfma(f2(-wr.x, -wr.x), q0, UV);           // exact remainder
-    return padd(pfma(rem, rr, q0), f2(0.5f, 0.5f));
+    if constexpr (WZ) {
+        const float2 wr = bp_w_r<true>(t, rc, az, P10);
+        return padd(bp_quotient2<true>(UV, wr.x, Recip{wr.y, 0.0f}), f2(0.5f, 0.5f));
+    }
+    return padd(bp_quotient2<EXACT>(UV, t.W, rc), f2(0.5f, 0.5f));
 }
 
 // The BPCore axis value (i - (n-1)/2) * pitch (BPCore.cpp:47-66).

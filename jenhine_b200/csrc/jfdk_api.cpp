@@ -251,6 +251,19 @@ BPParams bp_params(const jfdk_ctx* c) {
     return b;
 }
 
+// How the backprojection's matrices make a sample's place depend on z.
+void classify_geometry(jfdk_ctx* c) {
+    c->w_depends_on_z = c->u_depends_on_z = false;
+    for (int v = 0; v < c->nviews; ++v) {
+        if (c->ptms[(size_t)v * 12 + 10] != 0.0f) c->w_depends_on_z = true;
+        if (c->ptms[(size_t)v * 12 + 2] != 0.0f) c->u_depends_on_z = true;
+    }
+}
+
+Geo geometry(const jfdk_ctx* c) {
+    return c->w_depends_on_z ? kGeoWZ : c->u_depends_on_z ? kGeoWConst : kGeoIdeal;
+}
+
 // Slices per thread: the option, else 16 in the mixed form when W does not
 // depend on z and the volume holds at least 8 waves of 16-slice tiles (5
 // CTAs per SM), 8 otherwise.  16 slices halve the mixed loop's per-view work
@@ -348,10 +361,10 @@ jfdk_status run_bp_on(jfdk_ctx* c, BPParams b, bool finalize, cudaStream_t s) {
     if (mixed(c)) {
         b.qh = reinterpret_cast<const uint2*>(c->d_q4);
         b.qscale = c->d_qscale;
-        JFDK_LAUNCH(c, launch_bp_mixed(b, finalize, c->w_depends_on_z, bp_zpt(c), bp_tile(c), s), "backprojection");
+        JFDK_LAUNCH(c, launch_bp_mixed(b, finalize, geometry(c), bp_zpt(c), bp_tile(c), s), "backprojection");
         return JFDK_OK;
     }
-    JFDK_LAUNCH(c, launch_bp(b, finalize, c->opt_bp_exact != 0, c->w_depends_on_z, bp_zpt(c), bp_tile(c), s),
+    JFDK_LAUNCH(c, launch_bp(b, finalize, c->opt_bp_exact != 0, geometry(c), bp_zpt(c), bp_tile(c), s),
                 "backprojection");
     return JFDK_OK;
 }
@@ -578,8 +591,7 @@ jfdk_status jfdk_create(jfdk_ctx** out, const jfdk_scan_params* scan, const jfdk
     c->groups = (c->nviews + 8) / 9;
     c->ct_scale = recon->ct_norm0 * 1000.f / recon->mu_water;  // CTNumCore.cpp:24
     c->ptms.assign(h_ptms, h_ptms + (size_t)c->nviews * 12);
-    for (int v = 0; v < c->nviews; ++v)
-        if (c->ptms[(size_t)v * 12 + 10] != 0.0f) c->w_depends_on_z = true;
+    classify_geometry(c);
 
     int dev = 0;
     JFDK_CUDA(c, cudaGetDevice(&dev), "cudaGetDevice");
@@ -1177,9 +1189,7 @@ jfdk_status jfdk_set_bp_geometry(jfdk_ctx* c, const float* h_ptms) {
     if (!c || !h_ptms) return fail(c, JFDK_ERR_INVALID, "set_bp_geometry: bad argument");
     c->ptms.assign(h_ptms, h_ptms + (size_t)c->nviews * 12);
     c->wvol_state = 0;   // the normalisation weights follow the geometry
-    c->w_depends_on_z = false;
-    for (int v = 0; v < c->nviews; ++v)
-        if (c->ptms[(size_t)v * 12 + 10] != 0.0f) c->w_depends_on_z = true;
+    classify_geometry(c);
     JFDK_CUDA(c, cudaMemcpyAsync(c->d_ptm, c->ptms.data(), sizeof(float) * c->ptms.size(), cudaMemcpyHostToDevice,
                                  c->stream),
               "projection matrices upload");

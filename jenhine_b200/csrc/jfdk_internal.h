@@ -40,7 +40,15 @@ std::string build_host_operators(const jfdk_scan_params& scan, const jfdk_recon_
 constexpr int kBPTileX = 4;
 constexpr int kBPTileY = 32;
 
-// Parameters of the backprojection kernel (bp.cu).
+// How a sample's place depends on the slice (rows of the 3x4 matrices: U, V, W
+// = P (x, y, z, 1), u = U / W, v = V / W).
+enum Geo {
+    kGeoIdeal = 0,    // P[2] = P[10] = 0 in every view: u is the same in every slice (an untilted circular orbit)
+    kGeoWConst = 1,   // P[10] = 0 in every view: W is
+    kGeoWZ = 2        // W depends on z
+};
+
+// Parameters of the backprojection kernel (bp_body.cuh).
 struct BPParams {
     const float4* q4;        // quads, [slots][rows][U]: (p[r][c], p[r+1][c], p[r][c+1] - p[r][c], p[r+1][c+1] - p[r+1][c])
     const float2* tw;        // [views][U] taper pairs (w[c], RN(w[c+1] - w[c])), w[U] = 0
@@ -85,7 +93,11 @@ struct BatchScan {
 // Launchers (return cudaError_t of the launch).
 // zpt: slices per thread (4, 8 or 16); tile_x: CTA width in x, 4, 8 or 32
 // (CTAs of 128 threads; other values and 16-slice tiles take 4).
-cudaError_t launch_bp(const BPParams& p, bool finalize, bool exact, bool w_depends_on_z, int zpt, int tile_x,
+cudaError_t launch_bp_fast(const BPParams& p, bool finalize, Geo geo, int zpt, int tile_x, cudaStream_t s);
+cudaError_t launch_bp_exact(const BPParams& p, bool finalize, Geo geo, int zpt, int tile_x, cudaStream_t s);
+// The launch of frames with more than 4 GB of records (both forms).
+cudaError_t launch_bp_wide(const BPParams& p, bool finalize, bool exact, bool mixed_form, Geo geo, int zpt, cudaStream_t s);
+cudaError_t launch_bp(const BPParams& p, bool finalize, bool exact, Geo geo, int zpt, int tile_x,
                       cudaStream_t s);
 // The FP32 form's normalisation weights of every voxel of the volume over
 // every view of the rotation (p.v0 = 0, p.nv = all views, slices
@@ -108,6 +120,12 @@ struct BatchSlots {
 };
 // All tiles of nscans scans in one persistent launch of `ctas` CTAs (the
 // SMs' resident CTAs); *counter is the work-list cursor (cleared here).
+cudaError_t launch_bp_batch_fp32(const BatchSlots& t, int nscans, unsigned total, bool wz, bool wv, bool deep,
+                                 unsigned* counter, int ctas, cudaStream_t s);
+cudaError_t launch_bp_batch_mixed(const BatchSlots& t, int nscans, unsigned total, bool wz, bool wv, bool deep,
+                                  unsigned* counter, int ctas, cudaStream_t s);
+cudaError_t bp_batch_resident_fp32(bool wz, bool wv, bool deep, int* per_sm);
+cudaError_t bp_batch_resident_mixed(bool wz, bool wv, bool deep, int* per_sm);
 cudaError_t launch_bp_batch(const BatchSlots& t, int nscans, unsigned total_tiles, bool mixed_form, bool wz,
                             bool wv, unsigned* counter, int ctas, cudaStream_t s);
 // CTAs of a full persistent wave: SMs x resident CTAs per SM.
@@ -115,7 +133,7 @@ cudaError_t bp_batch_ctas(bool mixed_form, bool wz, bool wv, bool deep, int* cta
 // The context's backprojection store for every view (allocated if missing).
 jfdk_status ensure_store(jfdk_ctx* c);
 // Mixed-precision form: FP16 footprints with a per-view scale (qh, qscale).
-cudaError_t launch_bp_mixed(const BPParams& p, bool finalize, bool w_depends_on_z, int zpt, int tile_x,
+cudaError_t launch_bp_mixed(const BPParams& p, bool finalize, Geo geo, int zpt, int tile_x,
                             cudaStream_t s);
 // absmax[f] = bit pattern of max |plain[f][...]| over each of nv frames.
 cudaError_t launch_frame_absmax(const float* plain, long long frame, int nv, unsigned* absmax, cudaStream_t s);
@@ -287,6 +305,7 @@ struct jfdk_ctx {
     std::vector<float> ptms;
     jfdk::HostOperators ops;
     bool w_depends_on_z = false;  // some view has P[10] != 0
+    bool u_depends_on_z = false;  // some view has P[2] != 0
 
     // device constants
     float* d_ptm = nullptr;
