@@ -36,7 +36,9 @@ class FDKFunction(torch.autograd.Function):
             engine.bp_accumulate(q[v0:v0 + chunk], v0)
         vol = engine.finalize(apply_ctnum=False, device=p.device)
         ctx.engine, ctx.chunk = engine, chunk
-        ctx.dptm = torch.from_numpy(ptm_derivatives(P0, th).astype(np.float32)).to(p.device)
+        # formed while the kernels above run, and uploaded without waiting for them
+        dptm = torch.from_numpy(ptm_derivatives(P0, th).astype(np.float32))
+        ctx.dptm = dptm.pin_memory().to(p.device, non_blocking=True)
         ctx.theta_like = (theta.device, theta.dtype)
         ctx.save_for_backward(q, vol)
         return vol

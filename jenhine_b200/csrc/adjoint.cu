@@ -45,8 +45,12 @@ __global__ void residual_over_weight_kernel(const float* __restrict__ vol_bar, c
 // Quad-space adjoint: Qbar[view - v0][iv][iu] += rt * (bilinear weights).
 template <int ZPT, bool WZ>
 __global__ void __launch_bounds__(256) bp_adjoint_kernel(AdjParams p) {
-    const int x = blockIdx.x * 32 + threadIdx.x;
-    const int y = blockIdx.y * 8 + threadIdx.y;
+#ifndef AX
+#define AX 32
+#endif
+    const int tid0 = threadIdx.y * 32 + threadIdx.x;
+    const int x = blockIdx.x * AX + tid0 % AX;
+    const int y = blockIdx.y * (256 / AX) + tid0 / AX;
     const int zb = blockIdx.z * ZPT;
     if (x >= p.X || y >= p.Y) return;
     const float ax = bp_axis(x, p.X, p.pxy), ay = bp_axis(y, p.Y, p.pxy);
@@ -272,10 +276,11 @@ cudaError_t launch_residual_over_weight(const float* vol_bar, const float* cnt, 
 cudaError_t launch_bp_adjoint(const AdjParams& p, bool wz, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(p.qbar, 0, sizeof(float4) * (size_t)p.nv * p.q_frame, s);
     if (e != cudaSuccess) return e;
+    const dim3 g((p.X + AX - 1) / AX, (p.Y + 256 / AX - 1) / (256 / AX), (p.Z + kAdjZpt - 1) / kAdjZpt);
     if (wz)
-        bp_adjoint_kernel<kAdjZpt, true><<<bp_grid<kAdjZpt>(p), dim3(32, 8), 0, s>>>(p);
+        bp_adjoint_kernel<kAdjZpt, true><<<g, dim3(32, 8), 0, s>>>(p);
     else
-        bp_adjoint_kernel<kAdjZpt, false><<<bp_grid<kAdjZpt>(p), dim3(32, 8), 0, s>>>(p);
+        bp_adjoint_kernel<kAdjZpt, false><<<g, dim3(32, 8), 0, s>>>(p);
     return cudaGetLastError();
 }
 
