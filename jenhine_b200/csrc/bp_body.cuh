@@ -105,79 +105,24 @@ struct GridTileHeld {
 };
 
 // Whether every voxel of the CTA's tile samples every view of the launch
-// inside the detector, so that the view loop may leave out the range test
-// (two compares and two selects of a sample's 28 instructions in the FP32
-// form, two minima in the mixed one).  0 <= u <= U - 1, 0 <= v <= V - 1 and
-// W > 0 are linear in the voxel's place once multiplied by W, so the least
-// value over the tile's box is the one at its centre minus the coefficients'
-// moduli times the half extents: five such values per view, the views dealt
-// over the CTA's threads (under 0.5 % of the loop's work, whatever the
-// sizes).  The margin, 2^-16 of the sum of the terms' moduli, is far above
-// what the rounded coordinates can be off (a few 2^-24 of that sum, 16 steps
-// of it in the mixed form), so a tile that passes has no sample that the
-// range test would turn down, and the sums are the same bit for bit.  Frames
-// of more than 2^23 records are not taken (their record index is not exact
-// in a float, below).  Every thread of the CTA calls it.
+// inside the detector (box_inside), so that the view loop may leave out the
+// range test (two compares and two selects of a sample's 28 instructions in the
+// FP32 form, two minima in the mixed one).  The views are dealt over the CTA's
+// threads: under 0.5 % of the loop's work, whatever the sizes.  Frames of more
+// than 2^23 records are not taken (their record index is not exact in a float,
+// below).  Every thread of the CTA calls it.
 template <int ZPT, class Tile>
 __device__ __forceinline__ bool tile_inside(const BPParams& p, const Tile& tile) {
     bool ok = (long long)p.U * p.V <= (1LL << 23);
     if (ok) {
         const int x = tile.bx() * Tile::kX, y = tile.by() * Tile::kY, z = p.z_begin + tile.bz() * ZPT;
-        const float x0 = bp_axis(x, p.X, p.pxy), x1 = bp_axis(min(x + Tile::kX, p.X) - 1, p.X, p.pxy);
-        const float y0 = bp_axis(y, p.Y, p.pxy), y1 = bp_axis(min(y + Tile::kY, p.Y) - 1, p.Y, p.pxy);
-        const float z0 = bp_axis(z, p.Z, p.pz), z1 = bp_axis(z + ZPT - 1, p.Z, p.pz);   // all slices a thread walks
-        const float cx = 0.5f * (x0 + x1), cy = 0.5f * (y0 + y1), cz = 0.5f * (z0 + z1);
-        const float hx = 0.5f * fabsf(x1 - x0), hy = 0.5f * fabsf(y1 - y0), hz = 0.5f * fabsf(z1 - z0);
-        const float mx = fmaxf(fabsf(x0), fabsf(x1)), my = fmaxf(fabsf(y0), fabsf(y1)), mz = fmaxf(fabsf(z0), fabsf(z1));
-        // least value of a r + b r2 (rows of the matrix) over the box, against the margin
-        auto clear = [&](const float4& r, const float4& w, float a, float b, float lim) {
-            const float kx = fmaf(a, r.x, b * w.x), ky = fmaf(a, r.y, b * w.y), kz = fmaf(a, r.z, b * w.z);
-            const float f = fmaf(kx, cx, fmaf(ky, cy, fmaf(kz, cz, fmaf(a, r.w, b * w.w))));
-            const float h = fmaf(fabsf(kx), hx, fmaf(fabsf(ky), hy, fabsf(kz) * hz));
-            const float m = fmaf(fmaf(lim, fabsf(w.x), fabsf(r.x)), mx,
-                                 fmaf(fmaf(lim, fabsf(w.y), fabsf(r.y)), my,
-                                      fmaf(fmaf(lim, fabsf(w.z), fabsf(r.z)), mz, fmaf(lim, fabsf(w.w), fabsf(r.w)))));
-            return f - h > 0x1p-16f * m;   // false for NaN
-        };
-        const float ul = (float)p.U, vl = (float)p.V;
+        const VoxelBox box(bp_axis(x, p.X, p.pxy), bp_axis(min(x + Tile::kX, p.X) - 1, p.X, p.pxy),
+                           bp_axis(y, p.Y, p.pxy), bp_axis(min(y + Tile::kY, p.Y) - 1, p.Y, p.pxy),
+                           bp_axis(z, p.Z, p.pz), bp_axis(z + ZPT - 1, p.Z, p.pz));   // all slices a thread walks
         const int tid = threadIdx.y * Tile::kX + threadIdx.x;
-        for (int n = tid; n < p.nv; n += kBPThreads) {
-            const float4* P4 = reinterpret_cast<const float4*>(p.ptm + (size_t)(p.v0 + n) * 12);
-            const float4 r0 = __ldg(P4), r1 = __ldg(P4 + 1), r2 = __ldg(P4 + 2);
-            ok = ok && clear(r2, r2, 1.0f, 0.0f, 1.0f) && clear(r0, r2, 1.0f, 0.5f, ul) &&
-                 clear(r0, r2, -1.0f, ul - 1.5f, ul) && clear(r1, r2, 1.0f, 0.5f, vl) &&
-                 clear(r1, r2, -1.0f, vl - 1.5f, vl);
-        }
+        for (int n = tid; n < p.nv; n += kBPThreads) ok = ok && box_inside(box, p.ptm + (size_t)(p.v0 + n) * 12, p.U, p.V);
     }
     return __syncthreads_and(ok);
-}
-
-// Record loads.  The address is formed from a 32-bit byte offset, a shift on
-// the integer pipe, beside the view's base address: a 64-bit multiply-add
-// (IMAD.WIDE) instead takes two cycles of the FMA pipe, which is what bounds
-// the view loop (71 % busy; c2: 125.3 -> 119.3 ms FP32, 91.4 -> 82.3 ms
-// mixed).  WIDE: frames of more than 4 GB of records, and the batch kernel,
-// keep the 64-bit form.
-template <bool WIDE, class T>
-__device__ __forceinline__ T load_at(const T* frame, unsigned idx) {
-    if constexpr (WIDE) return __ldg(frame + idx);
-    return __ldg(reinterpret_cast<const T*>(reinterpret_cast<size_t>(frame) + idx * (unsigned)sizeof(T)));
-}
-
-// The record of integer column and row (as floats; tx = 2^23 + column) in a
-// frame of at most 2^23 records: 2^23 + row U + column is exact in a float,
-// and its bit pattern is the record's index above that of 2^23.  One FFMA in
-// place of two integer subtractions and a multiply-add; the constant part of
-// the shifted pattern is taken off the frame's address (record_base).
-template <class T>
-__device__ __forceinline__ T load_record(size_t base, float tx, float row, float Uf) {
-    const unsigned off = __float_as_uint(fmaf(row, Uf, tx)) * (unsigned)sizeof(T);   // mod 2^32
-    return __ldg(reinterpret_cast<const T*>(base + off));
-}
-
-template <class T>
-__device__ __forceinline__ size_t record_base(const T* frame) {
-    return reinterpret_cast<size_t>(frame) - (unsigned)kMagicBits * (unsigned)sizeof(T);
 }
 
 // The tile's (sum, weight) pairs: normalised, CT numbers, stored (FINALIZE),

@@ -151,20 +151,85 @@ __device__ __forceinline__ float2 bp_w_r(const XYTerms& t, const Recip& rc, floa
 
 // (u, v) of the sample at slice coordinate az.  WZ: W and its reciprocal are
 // the slice's, and the quotient is Markstein's (rl would cost two operations
-// a sample to save one).
+// a sample to save one).  w_r, quot: also W with its
+// reciprocal, and the quotients.
 template <bool EXACT, bool WZ>
-__device__ __forceinline__ float2 bp_uv(const XYTerms& t, const Recip& rc, float az, float P2, float P6, float P10) {
+__device__ __forceinline__ float2 bp_uv(const XYTerms& t, const Recip& rc, float az, float P2, float P6, float P10,
+                                        float2* w_r = nullptr, float2* quot = nullptr) {
     const float2 UV = f2(__fadd_rn(t.U, __fmul_rn(az, P2)), __fadd_rn(t.V, __fmul_rn(az, P6)));
-    if constexpr (WZ) {
-        const float2 wr = bp_w_r<true>(t, rc, az, P10);
-        return padd(bp_quotient2<true>(UV, wr.x, Recip{wr.y, 0.0f}), f2(0.5f, 0.5f));
-    }
-    return padd(bp_quotient2<EXACT>(UV, t.W, rc), f2(0.5f, 0.5f));
+    const float2 wr = bp_w_r<WZ>(t, rc, az, P10);
+    if (w_r) *w_r = wr;
+    const float2 q = WZ ? bp_quotient2<true>(UV, wr.x, Recip{wr.y, 0.0f}) : bp_quotient2<EXACT>(UV, t.W, rc);
+    if (quot) *quot = q;
+    return padd(q, f2(0.5f, 0.5f));
 }
 
 // The BPCore axis value (i - (n-1)/2) * pitch (BPCore.cpp:47-66).
 __device__ __forceinline__ float bp_axis(int i, int n, float pitch) {
     return __fmul_rn(__fadd_rn(-((float)n - 1.0f) / 2.0f, (float)i), pitch);
+}
+
+// Record loads.  The address is formed from a 32-bit byte offset, a shift on
+// the integer pipe, beside the view's base address: a 64-bit multiply-add
+// (IMAD.WIDE) instead takes two cycles of the FMA pipe, which is what bounds
+// the view loop (71 % busy; c2: 125.3 -> 119.3 ms FP32, 91.4 -> 82.3 ms
+// mixed).  WIDE: frames of more than 4 GB of records, and the batch kernel,
+// keep the 64-bit form.
+template <bool WIDE, class T>
+__device__ __forceinline__ T load_at(const T* frame, unsigned idx) {
+    if constexpr (WIDE) return __ldg(frame + idx);
+    return __ldg(reinterpret_cast<const T*>(reinterpret_cast<size_t>(frame) + idx * (unsigned)sizeof(T)));
+}
+
+// The record of integer column and row (as floats; tx = 2^23 + column) in a
+// frame of at most 2^23 records: 2^23 + row U + column is exact in a float,
+// and its bit pattern is the record's index above that of 2^23.  One FFMA in
+// place of two integer subtractions and a multiply-add; the constant part of
+// the shifted pattern is taken off the frame's address (record_base).
+template <class T>
+__device__ __forceinline__ T load_record(size_t base, float tx, float row, float Uf) {
+    const unsigned off = __float_as_uint(fmaf(row, Uf, tx)) * (unsigned)sizeof(T);   // mod 2^32
+    return __ldg(reinterpret_cast<const T*>(base + off));
+}
+
+template <class T>
+__device__ __forceinline__ size_t record_base(const T* frame) {
+    return reinterpret_cast<size_t>(frame) - (unsigned)kMagicBits * (unsigned)sizeof(T);
+}
+
+// A box of voxels: centre, half extents and largest moduli of its coordinates.
+struct VoxelBox {
+    float cx, cy, cz, hx, hy, hz, mx, my, mz;
+    __device__ VoxelBox(float x0, float x1, float y0, float y1, float z0, float z1)
+        : cx(0.5f * (x0 + x1)), cy(0.5f * (y0 + y1)), cz(0.5f * (z0 + z1)), hx(0.5f * fabsf(x1 - x0)),
+          hy(0.5f * fabsf(y1 - y0)), hz(0.5f * fabsf(z1 - z0)), mx(fmaxf(fabsf(x0), fabsf(x1))),
+          my(fmaxf(fabsf(y0), fabsf(y1))), mz(fmaxf(fabsf(z0), fabsf(z1))) {}
+};
+
+// Whether every voxel of the box samples the view of matrix P inside a U x V
+// detector, in front of the source.  0 <= u <= U - 1, 0 <= v <= V - 1 and W > 0
+// are linear in the voxel's place once multiplied by W, so the least value over
+// the box is the one at its centre minus the coefficients' moduli times the
+// half extents: five such values.  The margin, 2^-16 of the sum of the terms'
+// moduli, is far above what the rounded coordinates can be off (a few 2^-24 of
+// that sum, 16 steps of it in the mixed form), so no sample of a box that
+// passes would be turned down by the range test.
+__device__ __forceinline__ bool box_inside(const VoxelBox& b, const float* P, int U, int V) {
+    const float4* P4 = reinterpret_cast<const float4*>(P);
+    const float4 r0 = __ldg(P4), r1 = __ldg(P4 + 1), r2 = __ldg(P4 + 2);
+    // least value of k r + l r2 (rows of the matrix) over the box, against the margin
+    auto clear = [&](const float4& r, float k, float l, float lim) {
+        const float kx = fmaf(k, r.x, l * r2.x), ky = fmaf(k, r.y, l * r2.y), kz = fmaf(k, r.z, l * r2.z);
+        const float f = fmaf(kx, b.cx, fmaf(ky, b.cy, fmaf(kz, b.cz, fmaf(k, r.w, l * r2.w))));
+        const float h = fmaf(fabsf(kx), b.hx, fmaf(fabsf(ky), b.hy, fabsf(kz) * b.hz));
+        const float m = fmaf(fmaf(lim, fabsf(r2.x), fabsf(r.x)), b.mx,
+                             fmaf(fmaf(lim, fabsf(r2.y), fabsf(r.y)), b.my,
+                                  fmaf(fmaf(lim, fabsf(r2.z), fabsf(r.z)), b.mz, fmaf(lim, fabsf(r2.w), fabsf(r.w)))));
+        return f - h > 0x1p-16f * m;   // false for NaN
+    };
+    const float ul = (float)U, vl = (float)V;
+    return clear(r2, 1.0f, 0.0f, 1.0f) && clear(r0, 1.0f, 0.5f, ul) && clear(r0, -1.0f, ul - 1.5f, ul) &&
+           clear(r1, 1.0f, 0.5f, vl) && clear(r1, -1.0f, vl - 1.5f, vl);
 }
 
 }  // namespace

@@ -530,7 +530,7 @@ void jfdk_destroy(jfdk_ctx* c) {
     dev_free(c, c->d_plain);
     dev_free(c, c->d_q4); dev_free(c, c->d_qscale); dev_free(c, c->d_absmax);
     dev_free(c, c->d_sum); dev_free(c, c->d_cnt); dev_free(c, c->d_raw_stage); dev_free(c, c->d_hu_stage);
-    dev_free(c, c->d_Tt); dev_free(c, c->d_rt); dev_free(c, c->d_qadj); dev_free(c, c->d_partial);
+    dev_free(c, c->d_Tt); dev_free(c, c->d_qadj); dev_free(c, c->d_partial);
     dev_free(c, c->d_dptm);
     dev_free(c, c->d_wvol);
     for (auto& e : c->ev)
@@ -1159,23 +1159,15 @@ jfdk_status deriv_check(jfdk_ctx* c, const char* what) {
     return JFDK_OK;
 }
 
-jfdk_status ensure_rt(jfdk_ctx* c, const float* d_vol_bar) {
-    const size_t n = (size_t)c->X * c->Y * c->Z;
-    if (!c->d_rt) {
-        jfdk_status st = dev_alloc(c, &c->d_rt, n, "the adjoint residual");
-        if (st) return st;
-    }
-    JFDK_LAUNCH(c, launch_residual_over_weight(d_vol_bar, c->d_cnt, n, c->d_rt, c->stream), "residual / weight");
-    return JFDK_OK;
-}
-
-AdjParams adj_params(const jfdk_ctx* c, int v0, int nv) {
+AdjParams adj_params(const jfdk_ctx* c, const float* d_vol_bar, int v0, int nv) {
     AdjParams a{};
     a.ptm = c->d_ptm;
     a.v0 = v0; a.nv = nv; a.num_views = c->nviews;
     a.U = c->out_w; a.V = c->rows; a.X = c->X; a.Y = c->Y; a.Z = c->Z;
     a.pxy = c->pxy; a.pz = c->pz;
-    a.rt = c->d_rt;
+    a.vol_bar = d_vol_bar;
+    a.cnt = c->d_cnt;
+    a.sms = c->sms;
     a.q_frame = frame_px(c);
     a.tw = c->d_tw;
     return a;
@@ -1208,8 +1200,7 @@ jfdk_status jfdk_bp_adjoint(jfdk_ctx* c, const float* d_vol_bar, int v0, int nv,
         if ((st = dev_alloc(c, &c->d_qadj, (size_t)nv * frame_px(c), "the quad-space adjoint"))) return st;
         c->qadj_views = nv;
     }
-    if ((st = ensure_rt(c, d_vol_bar))) return st;
-    AdjParams a = adj_params(c, v0, nv);
+    AdjParams a = adj_params(c, d_vol_bar, v0, nv);
     a.qbar = c->d_qadj;
     JFDK_LAUNCH(c, launch_bp_adjoint(a, c->w_depends_on_z, c->stream), "backprojection adjoint");
     JFDK_LAUNCH(c, launch_unpack_adjoint(c->d_qadj, frame_px(c), nv, c->rows, c->out_w, c->d_tw, v0, c->nviews,
@@ -1251,8 +1242,7 @@ jfdk_status jfdk_geometry_gradient(jfdk_ctx* c, const float* d_q, int v0, int nv
     JFDK_LAUNCH(c, launch_pack_quads(d_q, frame_px(c), nv, c->rows, c->out_w, c->d_tw, v0, c->nviews, 1, c->d_q4,
                                      frame_px(c), 0, c->stream),
                 "packing projections");
-    if ((st = ensure_rt(c, d_vol_bar))) return st;
-    AdjParams a = adj_params(c, v0, nv);
+    AdjParams a = adj_params(c, d_vol_bar, v0, nv);
     a.q4 = c->d_q4;
     a.vol = d_vol;
     a.dptm = d_dptm;

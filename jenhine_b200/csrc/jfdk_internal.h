@@ -257,7 +257,8 @@ struct AdjParams {
     int v0, nv, num_views;   // views [v0, v0 + nv) of the rotation
     int U, V, X, Y, Z;
     float pxy, pz;
-    const float* rt;         // [Z][Y][X] vol_bar / weight
+    const float* vol_bar;    // [Z][Y][X] dL / dvol
+    const float* cnt;        // [Z][Y][X] the forward's weights: rt = vol_bar / cnt
     float4* qbar;            // adjoint out: quad space [nv][V][U]
     long long q_frame;       // V * U
     const float4* q4;        // gradient: the forward's tapered quads [nv][V][U]
@@ -265,8 +266,8 @@ struct AdjParams {
     const float* vol;        // gradient: the forward volume
     const float* dptm;       // gradient: [nv][6][12] dP / dtheta_j
     float* partial;          // gradient: [nv][ctas][6] scratch
+    int sms;
 };
-cudaError_t launch_residual_over_weight(const float* vol_bar, const float* cnt, size_t n, float* rt, cudaStream_t s);
 cudaError_t launch_bp_adjoint(const AdjParams& p, bool w_depends_on_z, cudaStream_t s);
 cudaError_t launch_unpack_adjoint(const float4* qbar, long long q_frame, int nv, int rows, int U, const float2* tw,
                                   int view0, int num_views, float* out, cudaStream_t s);
@@ -345,7 +346,6 @@ struct jfdk_ctx {
     float* d_hu_stage = nullptr; size_t hu_stage_bytes = 0;
     bool bp_has_views = false;
     // derivatives (allocated on demand)
-    float* d_rt = nullptr;                           // vol_bar / weight
     float4* d_qadj = nullptr; int qadj_views = 0;    // quad-space adjoint
     float* d_partial = nullptr; size_t partial_n = 0;
     float* d_dptm = nullptr; int dptm_views = 0;
