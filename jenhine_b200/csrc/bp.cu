@@ -37,6 +37,13 @@ __device__ __forceinline__ float view_scale(unsigned maxbits) {
     return ldexpf(1.0f, ilogbf(m) - 12);
 }
 
+// The packers write 16 or 8 bytes a pixel and are bound by that: a thread walks
+// kPackRows rows of its column, so that a row's samples serve as the upper
+// ones of one record and the lower ones of the one before, and the taper is
+// read once (a chunk of 32 frames of 768 x 768: 84.6 -> 57.4 us, 302 MB written at
+// 5.3 TB/s; mixed 99.4 -> 51.0).
+constexpr int kPackRows = 8;
+
 // Filtered frames -> mixed-precision records in slots [slot0, slot0 + nv),
 // tapered with the taper of rotation view (view0 + f) mod num_views; writes
 // that view's scale to scale[view].
@@ -46,53 +53,77 @@ __global__ void __launch_bounds__(256) pack_mixed_kernel(const float* __restrict
                                                          float* __restrict__ scale, uint2* __restrict__ qh,
                                                          long long q_frame, int slot0) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = blockIdx.y, f = blockIdx.z;
+    const int r0 = blockIdx.y * kPackRows, f = blockIdx.z;
     if (c >= U) return;
     const int view = (view0 + f) % num_views;
     const float s = view_scale(absmax[f]);
     const float inv = __fdiv_rn(1.0f, s);
-    if (r == 0 && c == 0) scale[view] = s;
-    uint2 rec = make_uint2(0u, 0u);   // the last row and column: samples not taken
-    if (c + 1 < U && r + 1 < rows) {
-        const float* src = plain + (size_t)f * plain_frame + (size_t)r * U + c;
-        const float w0 = tw[(size_t)view * U + c].x, w1 = tw[(size_t)view * U + c + 1].x;
-        // the tapered footprint over the view's scale (exact: inv a power of two)
-        const float a = (src[0] * w0) * inv, b = (src[1] * w1) * inv;
-        const float cc = (src[U] * w0) * inv, d = (src[U + 1] * w1) * inv;
-        const __half hp = __float2half_rn(a);
-        const float ap = __half2float(hp);
-        const __half hdx = __float2half_rn(b - ap), hdy = __float2half_rn(cc - ap);
-        const __half hdxy = __float2half_rn(d - (ap + __half2float(hdx) + __half2float(hdy)));
-        const __half2 h1 = __halves2half2(hp, hdx), h2 = __halves2half2(hdy, hdxy);
-        rec.x = *reinterpret_cast<const unsigned*>(&h1);
-        rec.y = *reinterpret_cast<const unsigned*>(&h2);
+    if (r0 == 0 && c == 0) scale[view] = s;
+    const bool right = c + 1 < U;
+    const float* src = plain + (size_t)f * plain_frame + (size_t)r0 * U + c;
+    uint2* dst = qh + (size_t)(slot0 + f) * q_frame + (size_t)r0 * U + c;
+    const float w0 = tw[(size_t)view * U + c].x, w1 = right ? tw[(size_t)view * U + c + 1].x : 0.0f;
+    // the tapered footprint over the view's scale (exact: inv a power of two)
+    float p[kPackRows + 1], q[kPackRows + 1];
+#pragma unroll
+    for (int i = 0; i <= kPackRows; ++i) {
+        const bool in = r0 + i < rows;
+        p[i] = in ? (src[(size_t)i * U] * w0) * inv : 0.0f;
+        q[i] = in && right ? (src[(size_t)i * U + 1] * w1) * inv : 0.0f;
     }
-    qh[(size_t)(slot0 + f) * q_frame + (size_t)r * U + c] = rec;
+#pragma unroll
+    for (int i = 0; i < kPackRows; ++i) {
+        if (r0 + i >= rows) break;
+        uint2 rec = make_uint2(0u, 0u);   // the last row and column: samples not taken
+        if (right && r0 + i + 1 < rows) {
+            const __half hp = __float2half_rn(p[i]);
+            const float ap = __half2float(hp);
+            const __half hdx = __float2half_rn(q[i] - ap), hdy = __float2half_rn(p[i + 1] - ap);
+            const __half hdxy = __float2half_rn(q[i + 1] - (ap + __half2float(hdx) + __half2float(hdy)));
+            const __half2 h1 = __halves2half2(hp, hdx), h2 = __halves2half2(hdy, hdxy);
+            rec.x = *reinterpret_cast<const unsigned*>(&h1);
+            rec.y = *reinterpret_cast<const unsigned*>(&h2);
+        }
+        dst[(size_t)i * U] = rec;
+    }
 }
 
-// Filtered frames -> tapered quads.  One thread per (row, column) of a frame:
-// the tapered values w[c] p[r][c], w[c] p[r+1][c], w[c+1] p[r][c+1],
-// w[c+1] p[r+1][c+1], each product rounded as InitView's in-place multiply
-// (BPCore.cpp:147-151), stored as (t00, t10, RN(t01 - t00), RN(t11 - t10)).
+// Filtered frames -> tapered quads: the tapered values w[c] p[r][c],
+// w[c] p[r+1][c], w[c+1] p[r][c+1], w[c+1] p[r+1][c+1], each product rounded as
+// InitView's in-place multiply (BPCore.cpp:147-151), stored as (t00, t10,
+// RN(t01 - t00), RN(t11 - t10)).
 __global__ void __launch_bounds__(256) pack_quads_kernel(const float* __restrict__ plain, long long plain_frame,
                                                          int rows, int U, const float2* __restrict__ tw,
                                                          int view0, int num_views, int apply_taper,
                                                          float4* __restrict__ q4, long long q4_frame, int slot0) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = blockIdx.y, f = blockIdx.z;
+    const int r0 = blockIdx.y * kPackRows, f = blockIdx.z;
     if (c >= U) return;
-    const float* s = plain + (size_t)f * plain_frame + (size_t)r * U + c;
-    const bool right = c + 1 < U, down = r + 1 < rows;
-    float p00 = s[0], p01 = right ? s[1] : 0.0f;
-    float p10 = down ? s[U] : 0.0f, p11 = (right && down) ? s[U + 1] : 0.0f;
+    const bool right = c + 1 < U;
+    const float* src = plain + (size_t)f * plain_frame + (size_t)r0 * U + c;
+    float4* dst = q4 + (size_t)(slot0 + f) * q4_frame + (size_t)r0 * U + c;
+    float w0 = 1.0f, w1 = 1.0f;
     if (apply_taper) {
         const float2* wv = tw + (size_t)((view0 + f) % num_views) * U;
-        const float w0 = wv[c].x, w1 = right ? wv[c + 1].x : 0.0f;
-        p00 = __fmul_rn(p00, w0); p10 = __fmul_rn(p10, w0);
-        p01 = __fmul_rn(p01, w1); p11 = __fmul_rn(p11, w1);
+        w0 = wv[c].x;
+        w1 = right ? wv[c + 1].x : 0.0f;
     }
-    q4[(size_t)(slot0 + f) * q4_frame + (size_t)r * U + c] =
-        make_float4(p00, p10, __fsub_rn(p01, p00), __fsub_rn(p11, p10));
+    float p[kPackRows + 1], q[kPackRows + 1];
+#pragma unroll
+    for (int i = 0; i <= kPackRows; ++i) {
+        const bool in = r0 + i < rows;
+        p[i] = in ? src[(size_t)i * U] : 0.0f;
+        q[i] = in && right ? src[(size_t)i * U + 1] : 0.0f;
+        if (apply_taper) {
+            p[i] = __fmul_rn(p[i], w0);
+            q[i] = __fmul_rn(q[i], w1);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kPackRows; ++i) {
+        if (r0 + i >= rows) break;
+        dst[(size_t)i * U] = make_float4(p[i], p[i + 1], __fsub_rn(q[i], p[i]), __fsub_rn(q[i + 1], p[i + 1]));
+    }
 }
 
 __global__ void finalize_kernel(const float* __restrict__ sum, const float* __restrict__ cnt, size_t n,
@@ -183,11 +214,22 @@ cudaError_t launch_frame_absmax(const float* plain, long long frame, int nv, uns
     return cudaGetLastError();
 }
 
+namespace {
+// Columns a packing CTA covers: 256, 128 or 64, the widest that leaves under a
+// quarter of the threads past the last column where one does.
+int pack_cta(int U) {
+    for (int t : {256, 128})
+        if ((U + t - 1) / t * t * 3 <= U * 4) return t;
+    return 64;
+}
+}  // namespace
+
 cudaError_t launch_pack_mixed(const float* plain, long long plain_frame, int nv, int rows, int U, const float2* tw,
                               int view0, int num_views, const unsigned* absmax, float* scale, uint2* qh,
                               long long q_frame, int slot0, cudaStream_t s) {
-    dim3 grid((U + 255) / 256, rows, nv);
-    pack_mixed_kernel<<<grid, 256, 0, s>>>(plain, plain_frame, rows, U, tw, view0, num_views, absmax, scale, qh,
+    const int cta = pack_cta(U);
+    dim3 grid((U + cta - 1) / cta, (rows + kPackRows - 1) / kPackRows, nv);
+    pack_mixed_kernel<<<grid, cta, 0, s>>>(plain, plain_frame, rows, U, tw, view0, num_views, absmax, scale, qh,
                                            q_frame, slot0);
     return cudaGetLastError();
 }
@@ -195,8 +237,9 @@ cudaError_t launch_pack_mixed(const float* plain, long long plain_frame, int nv,
 cudaError_t launch_pack_quads(const float* plain, long long plain_frame, int nv, int rows, int U, const float2* tw,
                               int view0, int num_views, int apply_taper, float4* q4, long long q4_frame, int slot0,
                               cudaStream_t s) {
-    dim3 grid((U + 255) / 256, rows, nv);
-    pack_quads_kernel<<<grid, 256, 0, s>>>(plain, plain_frame, rows, U, tw, view0, num_views, apply_taper, q4,
+    const int cta = pack_cta(U);
+    dim3 grid((U + cta - 1) / cta, (rows + kPackRows - 1) / kPackRows, nv);
+    pack_quads_kernel<<<grid, cta, 0, s>>>(plain, plain_frame, rows, U, tw, view0, num_views, apply_taper, q4,
                                            q4_frame, slot0);
     return cudaGetLastError();
 }
