@@ -245,11 +245,16 @@ jfdk_status jfdk_backproject_store(jfdk_ctx* ctx, int z0, int nz, float* d_hu, i
 enum {
     JFDK_OPT_BP_EXACT = 1,    /* FP32 form.  1: backprojection rounds every
                                  step like BPCore (bit-identical sums);
-                                 0 (default): the same sample coordinates
-                                 (correctly rounded quotients), lerps fused
-                                 into FMAs                                      */
+                                 0 (default): the same sample coordinates (but
+                                 for quotients that lie within 2^-47 of the
+                                 middle between two floats, rounded either
+                                 way), lerps fused into FMAs                    */
     JFDK_OPT_VIEW_CHUNK = 2,  /* views preprocessed + filtered per launch in
-                                 jfdk_reconstruct (default 32)                   */
+                                 jfdk_reconstruct (default: 32, or as many as
+                                 make the pixels of 32 frames of 768 x 768 when
+                                 frames are smaller and no
+                                 JFDK_OPT_DEVICE_MEMORY_LIMIT is set;
+                                 jfdk_reconstruct_host: 32)                      */
     JFDK_OPT_STAGE_TIMING = 3,/* 1: jfdk_reconstruct records CUDA events on its
                                  stream around each stage                        */
     JFDK_OPT_BP_ZPT = 4,      /* slices each backprojection thread keeps in
@@ -349,7 +354,8 @@ jfdk_status jfdk_geometry_gradient(jfdk_ctx* ctx, const float* d_q, int v0, int 
 /* Pick the backprojection's voxel tile (JFDK_OPT_BP_ZPT: 4 or 8 slices per
  * thread, and 16 in the mixed form; JFDK_OPT_BP_TILE: 4, 8 or 32 threads wide
  * in x, 128 per CTA, 16-slice tiles 4 wide) and
- * the filter stage's views per chunk (JFDK_OPT_VIEW_CHUNK: 16, 32 or 64) for
+ * the filter stage's views per chunk (JFDK_OPT_VIEW_CHUNK: 16, 32 or 64, 64 leaving the
+ * default where that is more) for
  * this context's shape by timing the candidates on the device (a 32-slice
  * slab, the first 128 views of zero frames).  Results are cached per shape in the process and, when
  * $JFDK_AUTOTUNE_CACHE names a file, appended to it and read back by later

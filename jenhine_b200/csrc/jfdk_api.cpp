@@ -251,6 +251,24 @@ BPParams bp_params(const jfdk_ctx* c) {
     return b;
 }
 
+// Views preprocessed and filtered per launch: the option, else 32, or as many
+// as make the pixels of 32 frames of 768 x 768 when frames are smaller: the
+// weighted rows and filtered frames of a chunk (150 MB there) pass from kernel
+// to kernel through L2, while 32 small frames leave each launch one or two
+// rounds of tiles (360 frames of 256 x 256: 477 us of filter stage in 12 chunks
+// of 32, 337 in two of 288 and 72; a mixed reconstruction 1070 -> 839 us).  A
+// context with a bound on its device memory keeps to 32.
+constexpr int kViewChunk = 32;
+int view_chunk(const jfdk_ctx* c) {
+    long long n = c->opt_view_chunk;
+    if (!n) {
+        n = kViewChunk;
+        if (c->mem_limit <= 0)
+            n = std::min(4096LL, std::max(n, 32LL * 768 * 768 / ((long long)c->rows * std::max(c->in_w, c->out_w))));
+    }
+    return (int)std::min<long long>(n, c->nviews);
+}
+
 // How the backprojection's matrices make a sample's place depend on z.
 void classify_geometry(jfdk_ctx* c) {
     c->w_depends_on_z = c->u_depends_on_z = false;
@@ -385,7 +403,7 @@ cudaError_t launch_ramp(jfdk_ctx* c, RampParams r) {
         case JFDK_RAMP_I8X14:
             r.row_scale = c->d_arow;
             r.b_scale = c->i8_scale;
-            return launch_ramp_i8(r, static_cast<const int8_t*>(a.hi),
+            return launch_ramp_i8(r, c->d_c64, static_cast<const int8_t*>(a.hi),
                                   (long long)(static_cast<const int8_t*>(a.lo) - static_cast<const int8_t*>(a.hi)),
                                   c->d_Ti8, (long long)c->out_w * a_pitch(c), c->d_i8mask, c->d_status, c->stream);
         default:
@@ -416,20 +434,28 @@ namespace jfdk {
 // Everything jfdk_reconstruct does before the backprojection, for the first
 // nviews views: per chunk of views raw -> weighted rows -> filtered frames
 // (L2-sized buffers) -> [z-filter] -> the BP store of the rotation.
-jfdk_status reconstruct_filter_stage(jfdk_ctx* c, const uint16_t* d_raw, int nviews, const cudaEvent_t* chunk_ready) {
+jfdk_status reconstruct_filter_stage(jfdk_ctx* c, const uint16_t* d_raw, int nviews, const cudaEvent_t* chunk_ready,
+                                     int chunk) {
     if (nviews < 0 || nviews > c->nviews) nviews = c->nviews;
-    return filter_stage_range(c, d_raw, 0, nviews, chunk_ready);
+    return filter_stage_range(c, d_raw, 0, nviews, chunk_ready, chunk);
 }
 
-jfdk_status filter_stage_range(jfdk_ctx* c, const uint16_t* d_raw, int vbeg, int vend, const cudaEvent_t* chunk_ready) {
+jfdk_status filter_stage_range(jfdk_ctx* c, const uint16_t* d_raw, int vbeg, int vend, const cudaEvent_t* chunk_ready,
+                               int chunk) {
     if (c->in_w != c->used_u && !compositing(c))
         return fail(c, JFDK_ERR_UNSUPPORTED,
                     "reconstruct: filter input width must be the frame width or twice it (compositing)");
     jfdk_status st = ensure_Q4(c, c->nviews);
     if (st) return st;
-    const int chunk = std::min(c->opt_view_chunk, c->nviews);
-    if ((st = ensure_A(c, (size_t)chunk * c->rows))) return st;
-    if ((st = ensure_plain(c, chunk))) return st;
+    if (!chunk) chunk = view_chunk(c);
+    st = ensure_A(c, (size_t)chunk * c->rows);
+    if (!st) st = ensure_plain(c, chunk);
+    if (st == JFDK_ERR_OOM && !c->opt_view_chunk && chunk > kViewChunk) {   // no room for the larger default
+        chunk = kViewChunk;
+        st = ensure_A(c, (size_t)chunk * c->rows);
+        if (!st) st = ensure_plain(c, chunk);
+    }
+    if (st) return st;
     const size_t frame = (size_t)c->scan.num_dets_u * c->scan.num_dets_v;
     for (int v0 = vbeg; v0 < vend; v0 += chunk) {
         const int nv = std::min(chunk, vend - v0);
@@ -526,7 +552,7 @@ void jfdk_destroy(jfdk_ctx* c) {
     dev_free(c, c->d_tinv_view); dev_free(c, c->d_cmask);
     dev_free(c, c->d_T); dev_free(c, c->d_Th); dev_free(c, c->d_Tl); dev_free(c, c->d_Tb); dev_free(c, c->d_Tf);
     dev_free(c, c->d_Ti8); dev_free(c, c->d_i8mask);
-    dev_free(c, c->d_status); dev_free(c, c->d_c); dev_free(c, c->d_A); dev_free(c, c->d_e); dev_free(c, c->d_arow);
+    dev_free(c, c->d_status); dev_free(c, c->d_c); dev_free(c, c->d_c64); dev_free(c, c->d_A); dev_free(c, c->d_e); dev_free(c, c->d_arow);
     dev_free(c, c->d_plain);
     dev_free(c, c->d_q4); dev_free(c, c->d_qscale); dev_free(c, c->d_absmax);
     dev_free(c, c->d_sum); dev_free(c, c->d_cnt); dev_free(c, c->d_raw_stage); dev_free(c, c->d_hu_stage);
@@ -704,6 +730,9 @@ jfdk_status jfdk_create(jfdk_ctx** out, const jfdk_scan_params* scan, const jfdk
             for (int j = 0; j < N; ++j)
                 for (int i = 0; i < P; ++i)
                     if (td[t * plane + (size_t)j * P + i]) mask[(size_t)(j / kI8TileN) * nk + i / kI8BlockK] |= (uint8_t)(1u << t);
+        const std::vector<double> c64(c->ops.c.begin(), c->ops.c.end());
+        if ((st = dev_alloc(c, &c->d_c64, c64.size(), "the edge response"))) return bail(st);
+        JFDK_CUDA(c, cudaMemcpyAsync(c->d_c64, c64.data(), sizeof(double) * c64.size(), cudaMemcpyHostToDevice, c->stream), "upload");
         if ((st = dev_alloc(c, &c->d_Ti8, td.size(), "the operator's digits"))) return bail(st);
         if ((st = dev_alloc(c, &c->d_i8mask, mask.size(), "the digit masks"))) return bail(st);
         JFDK_CUDA(c, cudaMemcpyAsync(c->d_Ti8, td.data(), td.size(), cudaMemcpyHostToDevice, c->stream), "upload");
@@ -786,7 +815,7 @@ jfdk_status jfdk_get_option(jfdk_ctx* c, int key, long long* value) {
     if (!c || !value) return JFDK_ERR_INVALID;
     switch (key) {
         case JFDK_OPT_BP_EXACT: *value = c->opt_bp_exact; return JFDK_OK;
-        case JFDK_OPT_VIEW_CHUNK: *value = c->opt_view_chunk; return JFDK_OK;
+        case JFDK_OPT_VIEW_CHUNK: *value = c->opt_view_chunk ? c->opt_view_chunk : view_chunk(c); return JFDK_OK;
         case JFDK_OPT_STAGE_TIMING: *value = c->opt_stage_timing; return JFDK_OK;
         case JFDK_OPT_BP_ZPT: *value = bp_zpt(c); return JFDK_OK;
         case JFDK_OPT_BP_TILE: *value = bp_zpt(c) == 16 ? kBPTileX : bp_tile(c); return JFDK_OK;
@@ -963,8 +992,12 @@ jfdk_status jfdk_filter_raw(jfdk_ctx* c, const uint16_t* d_raw, int v0, int nv, 
     if (c->in_w != c->used_u && !compositing(c))
         return fail(c, JFDK_ERR_UNSUPPORTED,
                     "filter_raw: filter input width must be the frame width or twice it (compositing)");
-    const int chunk = std::min(c->opt_view_chunk, c->nviews);
+    int chunk = std::min(view_chunk(c), nv);
     jfdk_status st = ensure_A(c, (size_t)chunk * c->rows);
+    if (st == JFDK_ERR_OOM && !c->opt_view_chunk && chunk > kViewChunk) {
+        chunk = kViewChunk;
+        st = ensure_A(c, (size_t)chunk * c->rows);
+    }
     if (st) return st;
     const size_t frame = (size_t)c->scan.num_dets_u * c->scan.num_dets_v;
     for (int a = v0; a < v0 + nv; a += chunk) {
@@ -1088,7 +1121,8 @@ jfdk_status jfdk_reconstruct_host(jfdk_ctx* c, const uint16_t* h_raw, float* h_h
         if ((st = dev_alloc(c, &c->d_hu_stage, hu_bytes / sizeof(float), "the output volume"))) return st;
         c->hu_stage_bytes = hu_bytes;
     }
-    const int chunk = std::min(c->opt_view_chunk, c->nviews);
+    // (chunks of the upload: small ones, so that filtering starts early)
+    const int chunk = std::min(c->opt_view_chunk ? c->opt_view_chunk : kViewChunk, c->nviews);
     const int nchunks = (c->nviews + chunk - 1) / chunk;
     const int zpt = bp_zpt(c);
     const int slab = (int)round_up((c->Z + kHostSlabs - 1) / kHostSlabs, zpt);
@@ -1116,7 +1150,7 @@ jfdk_status jfdk_reconstruct_host(jfdk_ctx* c, const uint16_t* h_raw, float* h_h
         if ((st = upload_chunk(c, h_raw, v0, std::min(chunk, c->nviews - v0), up))) return drain(st);
         JFDK_CUDA(c, cudaEventRecord(ev[k], c->copy_stream), "event");
     }
-    if ((st = jfdk::reconstruct_filter_stage(c, c->d_raw_stage, c->nviews, ev))) return drain(st);
+    if ((st = jfdk::reconstruct_filter_stage(c, c->d_raw_stage, c->nviews, ev, chunk))) return drain(st);
     if (timing) {
         JFDK_CUDA(c, cudaEventRecord(c->ev[1], c->stream), "event");
         JFDK_CUDA(c, cudaEventRecord(c->ev[2], c->stream), "event");
@@ -1307,6 +1341,13 @@ void tune_file_append(const std::string& key, const TuneChoice& t) {
     std::fclose(f);
 }
 
+// The tuned views per chunk; the largest candidate stands for "as many as the
+// frame size calls for" where that is more.
+void take_chunk(jfdk_ctx* c, int chunk) {
+    c->opt_view_chunk = 0;
+    if (chunk != 64 || view_chunk(c) <= 64) c->opt_view_chunk = chunk;
+}
+
 // The smaller of two timed runs after one warm-up run.
 template <class F>
 jfdk_status time_ms(jfdk_ctx* c, F&& run, float* ms) {
@@ -1341,7 +1382,7 @@ extern "C" jfdk_status jfdk_autotune(jfdk_ctx* c, int flags) {
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end() && !(flags & JFDK_AUTOTUNE_FORCE)) {
             c->opt_bp_zpt = it->second.zpt;
-            c->opt_view_chunk = it->second.chunk;
+            take_chunk(c, it->second.chunk);
             c->opt_bp_tile = it->second.tile;
             return JFDK_OK;
         }
@@ -1382,7 +1423,7 @@ extern "C" jfdk_status jfdk_autotune(jfdk_ctx* c, int flags) {
     c->opt_bp_zpt = best_z;
     c->opt_bp_tile = best_x;
     // views per chunk: the filter stage over the first views of zero frames
-    int best_c = c->opt_view_chunk;
+    int best_c = c->opt_view_chunk ? c->opt_view_chunk : kViewChunk;
     if (c->in_w == c->used_u) {   // (compositing reads conjugate frames of the whole rotation)
         const int nsub = std::min(c->nviews, 128);
         uint16_t* raw = nullptr;
@@ -1401,7 +1442,7 @@ extern "C" jfdk_status jfdk_autotune(jfdk_ctx* c, int flags) {
         dev_free(c, raw);
         if (st) return st;
     }
-    c->opt_view_chunk = best_c;
+    take_chunk(c, best_c);
     std::lock_guard<std::mutex> lk(g_tune_mutex);
     g_tune_cache[key] = {best_z, best_c, best_x};
     tune_file_append(key, g_tune_cache[key]);

@@ -248,7 +248,7 @@ float tf32_round_host(float x);
 // that are not all zero ([ceil(N / kI8TileN)][ceil(a_pitch / kI8BlockK)]).
 constexpr int kI8TileN = 64;
 constexpr int kI8BlockK = 128;
-cudaError_t launch_ramp_i8(const RampParams& p, const int8_t* A, long long a_plane, const int8_t* B,
+cudaError_t launch_ramp_i8(const RampParams& p, const double* c64, const int8_t* A, long long a_plane, const int8_t* B,
                            long long b_plane, const uint8_t* masks, int* status, cudaStream_t s);
 
 // Derivatives (adjoint.cu).
@@ -328,6 +328,7 @@ struct jfdk_ctx {
     float i8_scale = 1.0f;       // 2^F of the operator's digits
     float* d_czero = nullptr;    // [in_w] zeros
     float* d_c = nullptr;
+    double* d_c64 = nullptr;     // d_c in double (the int8 product's epilogue)
     int* d_status = nullptr;     // nonzero: a kernel's bounded wait gave up
 
     // device working storage (allocated on demand)
@@ -352,7 +353,7 @@ struct jfdk_ctx {
 
     // JFDK_OPT_* settings
     int opt_bp_exact = 0;
-    int opt_view_chunk = 32;
+    int opt_view_chunk = 0;      // 0: by the frame size (view_chunk)
     int opt_stage_timing = 0;
     int opt_bp_zpt = 0;          // 0: default (bp_zpt() in jfdk_api.cpp)
     int opt_bp_tile = 0;         // tile width in x: 4, 8 or 32; 0: default (4)
@@ -379,10 +380,11 @@ namespace jfdk {
 // chunk_ready (optional): one event per chunk of views; the stage waits for
 // chunk k's event before its first kernel (frames still in transfer).
 jfdk_status reconstruct_filter_stage(jfdk_ctx* c, const uint16_t* d_raw, int nviews,
-                                     const cudaEvent_t* chunk_ready = nullptr);
+                                     const cudaEvent_t* chunk_ready = nullptr, int chunk = 0);
 // The same for views [vbeg, vend) only (d_raw: the rotation's frames).
+// chunk: views per chunk (0: the context's own).
 jfdk_status filter_stage_range(jfdk_ctx* c, const uint16_t* d_raw, int vbeg, int vend,
-                               const cudaEvent_t* chunk_ready = nullptr);
+                               const cudaEvent_t* chunk_ready = nullptr, int chunk = 0);
 BPParams reconstruct_bp_params(const jfdk_ctx* c, float* d_hu, int16_t* d_hu16);
 // The finalizing backprojection of every view into d_hu, on stream s.
 jfdk_status reconstruct_bp(jfdk_ctx* c, float* d_hu, cudaStream_t s);

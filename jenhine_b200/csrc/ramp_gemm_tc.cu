@@ -310,13 +310,24 @@ __global__ void __launch_bounds__(kThreads, 1) ramp_tc_kernel(const __grid_const
 // are below 2^-30 of the leading one.
 //
 // Tile 128 rows x kI8TileN columns, K blocks of kI8BlockK bytes (128-byte
-// swizzle, whole 128-byte rows as the TMA reads best): per stage the four
-// row digit planes (one 3-D TMA load, 64 KB) and the operator digit planes
-// that are not all zero in this block (the host's mask; far from the
-// diagonal the leading bytes of the ramp are zero), up to 32 KB.  Two sets of four level accumulators of kI8TileN
+// swizzle, whole 128-byte rows as the TMA reads best): per stage the operator
+// digit planes that are not all zero in this block (the host's mask; far from
+// the diagonal the leading bytes of the ramp are zero), up to 32 KB, and the
+// row digit planes that meet one of them in a product, s <= 3 - the least such
+// t, up to 64 KB (the leading operator byte only reaches 10 columns from the
+// diagonal, the second 160).  Two sets of four level accumulators of kI8TileN
 // columns fill the tensor memory, so one tile's epilogue overlaps the next
 // tile's MMAs.
-constexpr int I8_BN = kI8TileN, I8_BK = kI8BlockK, I8_STAGES = 2, I8_LEVELS = 4, I8_PRODUCTS = 10;
+//
+// What bounded it was the products, not the loads (without them the tiles took
+// 155 us still, without the products 88): ten instructions of 64 columns per 32
+// bytes of K, each put together from tables by the one thread that issues.  A
+// row plane now meets all its operator planes in one instruction of up to 256
+// columns, four instead of ten.  A chunk of 32 frames of 768 x 768: 165 us,
+// 148 with the tables gone, 117 with the wide instructions, 108 with eight
+// epilogue warps instead of four (loads and waits alone take 57).
+constexpr int kI8EpilogueWarps = 8, kI8Threads = 32 * (2 + kI8EpilogueWarps);
+constexpr int I8_BN = kI8TileN, I8_BK = kI8BlockK, I8_STAGES = 2, I8_LEVELS = 4;
 constexpr int I8_ATILE = BM * I8_BK;                         // one row digit plane: 16 KB
 constexpr int I8_BTILE = I8_BN * I8_BK;                      // one operator digit plane: 8 KB
 constexpr int I8_STAGE_BYTES = kI8RowDigits * I8_ATILE + kI8OpDigits * I8_BTILE;
@@ -326,21 +337,16 @@ static_assert(2 * I8_ACC_COLS == 512, "two accumulator sets fill the tensor memo
 static_assert(I8_BK == 128 && I8_ATILE % 1024 == 0 && I8_BTILE % 1024 == 0 && I8_STAGE_BYTES % 1024 == 0,
               "128-byte swizzle atoms");
 static_assert(I8_SMEM_BYTES <= 227 * 1024, "shared memory");
-// (row byte, operator byte) of each product, by level; first[p]: the first
-// product of its level (starts the accumulator in the first K step)
-__constant__ const unsigned char kI8S[I8_PRODUCTS] = {0, 0, 1, 0, 1, 2, 0, 1, 2, 3};
-__constant__ const unsigned char kI8T[I8_PRODUCTS] = {0, 1, 0, 2, 1, 0, 3, 2, 1, 0};
-__constant__ const unsigned char kI8First[I8_PRODUCTS] = {1, 1, 0, 1, 0, 0, 1, 0, 0, 0};
+// D = S32, A = B = signed 8-bit, both K-major, M = 128, N columns.
+__device__ __forceinline__ uint32_t i8_idesc(int n) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}
 
-// D = S32, A = B = signed 8-bit, both K-major, M = 128, N = I8_BN.
-constexpr uint32_t kI8Idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(I8_BN >> 3) << 17) |
-                              ((uint32_t)(BM >> 4) << 24);
-
-__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
+__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc_n, uint32_t accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(kI8Idesc), "r"(accumulate));
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc_n), "r"(accumulate));
 }
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
@@ -350,13 +356,20 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
+// The double of a signed 32-bit integer's bits: 2^52 + 2^31 + a assembled in
+// place, less 2^52 + 2^31, one addition on the FP64 pipe.
+__device__ __forceinline__ double int_double(uint32_t a) {
+    return __hiloint2double(0x43300000, (int)(a ^ 0x80000000u)) - 4503601774854144.0;
+}
+
 struct I8Args {
     RampParams p;
+    const double* c64;       // p.c in double
     const uint8_t* masks;    // [tiles_n][nk]
     int* status;
 };
 
-__global__ void __launch_bounds__(kThreads, 1) ramp_i8_kernel(const __grid_constant__ CUtensorMap mapA,
+__global__ void __launch_bounds__(kI8Threads, 1) ramp_i8_kernel(const __grid_constant__ CUtensorMap mapA,
                                                                const __grid_constant__ CUtensorMap mapB,
                                                                I8Args args) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -380,7 +393,7 @@ __global__ void __launch_bounds__(kThreads, 1) ramp_i8_kernel(const __grid_const
     if (tid == 0) {
         abort_flag = 0;
         for (int s = 0; s < I8_STAGES; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(tfull(b), 1); mbar_init(tempty(b), 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(tfull(b), 1); mbar_init(tempty(b), kI8EpilogueWarps); }
         mbar_init(drain_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -397,10 +410,18 @@ __global__ void __launch_bounds__(kThreads, 1) ramp_i8_kernel(const __grid_const
     auto b_tile = [&](int s, int t) {
         return base + (uint32_t)(s * I8_STAGE_BYTES + kI8RowDigits * I8_ATILE + t * I8_BTILE);
     };
-    // operator digit planes used in K block kb of output tile nt: all of
-    // them in the first block (it starts every level's accumulator)
-    auto block_mask = [&](int nt, int kb) -> uint32_t {
-        return kb == 0 ? (1u << kI8OpDigits) - 1u : (uint32_t)__ldg(args.masks + (size_t)nt * nk + kb);
+    // operator digit planes that are not zero in K block kb of output tile nt
+    auto block_mask = [&](int nt, int kb) -> uint32_t { return (uint32_t)__ldg(args.masks + (size_t)nt * nk + kb); };
+    // the planes loaded: from the operator's leading nonzero one on, and all of
+    // them in the first block, whose products with the leading row plane start
+    // every level's accumulator
+    auto op_planes = [](uint32_t mask, int kb) -> uint32_t {
+        const uint32_t all = (1u << kI8OpDigits) - 1u;
+        return kb == 0 ? all : mask ? all << (__ffs(mask) - 1) & all : 0u;
+    };
+    auto row_planes = [](uint32_t mask, int kb) -> int {   // the leading so many of the rows'
+        const int n = mask ? kI8RowDigits - (__ffs(mask) - 1) : 0;
+        return kb == 0 && n == 0 ? 1 : n;
     };
 
     if (warp == 0) {
@@ -413,9 +434,10 @@ __global__ void __launch_bounds__(kThreads, 1) ramp_i8_kernel(const __grid_const
                 for (int kb = 0; kb < nk; ++kb, ++it) {
                     const int s = (int)(it % I8_STAGES);
                     if (it >= I8_STAGES && !mbar_wait(empty(s), ((it / I8_STAGES) - 1) & 1u, abort_v)) break;
-                    const uint32_t mask = block_mask(nt, kb);
-                    mbar_expect_tx(full(s), (uint32_t)(kI8RowDigits * I8_ATILE) + (uint32_t)__popc(mask) * I8_BTILE);
-                    tma_load_3d(a_tile(s), &mapA, kb * I8_BK, m0, 0, full(s));
+                    const uint32_t nz = block_mask(nt, kb), mask = op_planes(nz, kb);
+                    const int rows = row_planes(nz, kb);
+                    mbar_expect_tx(full(s), (uint32_t)rows * I8_ATILE + (uint32_t)__popc(mask) * I8_BTILE);
+                    for (int d = 0; d < rows; ++d) tma_load_3d(a_tile(s) + (uint32_t)d * I8_ATILE, &mapA, kb * I8_BK, m0, d, full(s));
                     for (int d = 0; d < kI8OpDigits; ++d)
                         if ((mask >> d) & 1u) tma_load_3d(b_tile(s, d), &mapB, kb * I8_BK, n0, d, full(s));
                 }
@@ -444,16 +466,21 @@ __global__ void __launch_bounds__(kThreads, 1) ramp_i8_kernel(const __grid_const
                     const uint32_t mask = block_mask(nt, kb);
                     if (!mbar_wait(full(s), (it / I8_STAGES) & 1u, abort_v)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    // Row plane i times the operator's planes j .. 3 - i, which
+                    // lie one behind the other as the levels' accumulators do:
+                    // one instruction of 64 (4 - i - j) columns.  The first
+                    // one starts every level.
+                    const uint64_t da = smem_desc(a_tile(s)), db = smem_desc(b_tile(s, 0));
+                    const int lead = mask ? __ffs(mask) - 1 : kI8OpDigits;
 #pragma unroll
                     for (int ks = 0; ks < I8_BK / 32; ++ks) {
-                        const uint32_t off = (uint32_t)ks * 32u;
 #pragma unroll
-                        for (int q = 0; q < I8_PRODUCTS; ++q) {
-                            if (!((mask >> kI8T[q]) & 1u)) continue;
-                            const uint32_t level = (uint32_t)(kI8S[q] + kI8T[q]);
-                            const uint64_t da = smem_desc(a_tile(s) + (uint32_t)kI8S[q] * I8_ATILE + off);
-                            const uint64_t db = smem_desc(b_tile(s, kI8T[q]) + off);
-                            mma_i8(acc + level * (uint32_t)I8_BN, da, db, (kb == 0 && ks == 0 && kI8First[q]) ? 0u : 1u);
+                        for (int i = 0; i < kI8RowDigits; ++i) {
+                            const bool start = i == 0 && ks == 0 && kb == 0;
+                            const int j = start ? 0 : lead, levels = I8_LEVELS - i - j;
+                            if (levels > 0)
+                                mma_i8(acc + (uint32_t)((i + j) * I8_BN), da + (uint64_t)((i * I8_ATILE + ks * 32) >> 4),
+                                       db + (uint64_t)((j * I8_BTILE + ks * 32) >> 4), i8_idesc(levels * I8_BN), start ? 0u : 1u);
                         }
                     }
                     mma_commit(empty(s));
@@ -466,8 +493,9 @@ __global__ void __launch_bounds__(kThreads, 1) ramp_i8_kernel(const __grid_const
             mbar_wait(drain_bar, 0, &dummy);
         }
     } else {
-        // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 ----
-        const int quarter = warp & 3;
+        // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31, two warps
+        // a quarter with half of the columns each ----
+        const int quarter = warp & 3, cols = (warp - 2) / 4 * (I8_BN / 2);
         uint32_t i = 0;
         for (int t = blockIdx.x; t < tiles && !*abort_v; t += gridDim.x, ++i) {
             const int b = (int)(i & 1u);
@@ -488,7 +516,7 @@ __global__ void __launch_bounds__(kThreads, 1) ramp_i8_kernel(const __grid_const
                 qrow = p.q + (size_t)vl * p.q_frame_stride + (size_t)row * p.q_pitch;
             }
 #pragma unroll 1
-            for (int c0 = 0; c0 < I8_BN; c0 += 16) {
+            for (int c0 = cols; c0 < cols + I8_BN / 2; c0 += 16) {
                 uint32_t r[I8_LEVELS][16];
 #pragma unroll
                 for (int l = 0; l < I8_LEVELS; ++l) {
@@ -507,12 +535,13 @@ __global__ void __launch_bounds__(kThreads, 1) ramp_i8_kernel(const __grid_const
                     float o[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        // exact: |acc_l| < 2^31, so |V| < 2^56
-                        long long v = (int)r[0][j];
+                        // |acc_l| < 2^31: exact up to the last sum, which rounds V once
+                        double v = int_double(r[I8_LEVELS - 1][j]);
 #pragma unroll
-                        for (int l = 1; l < I8_LEVELS; ++l) v = v * 256 + (int)r[l][j];
-                        const double cn = (double)__ldg(p.c + (n + j < p.N ? n + j : p.N - 1));
-                        o[j] = (float)fma((double)v, scale, cn * em);
+                        for (int l = I8_LEVELS - 2; l >= 0; --l)
+                            v = fma(int_double(r[l][j]), (double)(1 << 8 * (I8_LEVELS - 1 - l)), v);
+                        const double cn = __ldg(args.c64 + (n + j < p.N ? n + j : p.N - 1));
+                        o[j] = (float)fma(v, scale, cn * em);
                         if (n + j < p.N) amax = fmaxf(amax, fabsf(o[j]));
                     }
                     if (p.vec_store && n + 16 <= p.N) {
@@ -585,14 +614,14 @@ bool make_map(CUtensorMap* map, const void* ptr, int kind, int rows, int cols) {
 }
 
 // planes x rows x cols int8 (K-major planes, plane_bytes apart); box =
-// 128 bytes of K x box_rows rows x box_planes planes, 128-byte swizzle.
+// 128 bytes of K x box_rows rows of one plane, 128-byte swizzle.
 bool make_map_i8(CUtensorMap* map, const void* ptr, int planes, int rows, int cols, long long plane_bytes,
-                 int box_rows, int box_planes) {
+                 int box_rows) {
     EncodeFn enc = encoder();
     if (!enc) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)planes};
     const cuuint64_t strides[2] = {(cuuint64_t)cols, (cuuint64_t)plane_bytes};
-    const cuuint32_t box[3] = {(cuuint32_t)I8_BK, (cuuint32_t)box_rows, (cuuint32_t)box_planes};
+    const cuuint32_t box[3] = {(cuuint32_t)I8_BK, (cuuint32_t)box_rows, 1u};
     const cuuint32_t estr[3] = {1, 1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -632,15 +661,15 @@ cudaError_t launch_kind(const RampParams& p, const void* Ah, const void* Al, con
 
 }  // namespace
 
-cudaError_t launch_ramp_i8(const RampParams& p, const int8_t* A, long long a_plane, const int8_t* B,
+cudaError_t launch_ramp_i8(const RampParams& p, const double* c64, const int8_t* A, long long a_plane, const int8_t* B,
                            long long b_plane, const uint8_t* masks, int* status, cudaStream_t s) {
-    if (p.a_pitch % 16 != 0 || p.M < 1 || p.N < 1 || !p.row_scale || !masks) return cudaErrorInvalidValue;
+    if (p.a_pitch % 16 != 0 || p.M < 1 || p.N < 1 || !p.row_scale || !masks || !c64) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || a_plane % 16 ||
         b_plane % 16)
         return cudaErrorInvalidValue;
     CUtensorMap ma, mb;
-    if (!make_map_i8(&ma, A, kI8RowDigits, p.M, p.a_pitch, a_plane, BM, kI8RowDigits) ||
-        !make_map_i8(&mb, B, kI8OpDigits, p.N, p.a_pitch, b_plane, I8_BN, 1))
+    if (!make_map_i8(&ma, A, kI8RowDigits, p.M, p.a_pitch, a_plane, BM) ||
+        !make_map_i8(&mb, B, kI8OpDigits, p.N, p.a_pitch, b_plane, I8_BN))
         return cudaErrorInvalidValue;
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
@@ -650,8 +679,8 @@ cudaError_t launch_ramp_i8(const RampParams& p, const int8_t* A, long long a_pla
     if (attr != cudaSuccess) return attr;
     const int tiles = ((p.M + BM - 1) / BM) * ((p.N + I8_BN - 1) / I8_BN);
     const int grid = tiles < sm_count() ? tiles : sm_count();
-    I8Args a{p, masks, status};
-    ramp_i8_kernel<<<grid, kThreads, I8_SMEM_BYTES, s>>>(ma, mb, a);
+    I8Args a{p, c64, masks, status};
+    ramp_i8_kernel<<<grid, kI8Threads, I8_SMEM_BYTES, s>>>(ma, mb, a);
     return cudaGetLastError();
 }
 
