@@ -2,10 +2,8 @@
 //
 //   * the adjoint of the backprojector, vol = S q / C: with the weights C
 //     (the backprojected taper) fixed, q_bar = S^T (vol_bar / C) -- for every
-//     voxel and view the transposed bilinear weights of its sample point,
-//     scattered into "quad space" (the forward's tapered footprint records,
-//     one 16-byte vector atomic per sample) and folded back to detector
-//     pixels and multiplied by the taper;
+//     voxel and view the transposed bilinear weights of its sample point, summed
+//     in patches of the view in shared memory and multiplied by the taper;
 //   * the adjoint of the ramp filter, y = T (w o x) + c e(x) with
 //     e(x) = (x0 + x1 + x2) / 3 (or the last three for a mirrored filter):
 //     x_bar = w o (T^T y_bar) + (c . y_bar) / 3 on the edge samples;
@@ -28,74 +26,213 @@
 namespace jfdk {
 namespace {
 
-__device__ __forceinline__ void red_add_v4(float4* p, float4 v) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-                 : "memory");
-}
-
 // rt = vol_bar / C (0 where no view saw the voxel).
 __device__ __forceinline__ float residual(float vol_bar, float cnt) { return cnt != 0.0f ? vol_bar / cnt : 0.0f; }
 
 constexpr int kAdjZpt = 8;
 
-// Quad-space adjoint: Qbar[view - v0][iv][iu] += rt * (bilinear weights).
-template <int ZPT, bool WZ>
-__global__ void __launch_bounds__(256) bp_adjoint_kernel(AdjParams p) {
-    const int x = blockIdx.x * 32 + threadIdx.x;
-    const int y = blockIdx.y * 8 + threadIdx.y;
-    const int zb = blockIdx.z * ZPT;
-    if (x >= p.X || y >= p.Y) return;
-    const float ax = bp_axis(x, p.X, p.pxy), ay = bp_axis(y, p.Y, p.pxy);
-    const size_t plane = (size_t)p.X * p.Y, base = (size_t)y * p.X + x;
-    float az[ZPT], rt[ZPT];
-    bool any = false;
-#pragma unroll
-    for (int k = 0; k < ZPT; ++k) {
-        az[k] = bp_axis(zb + k, p.Z, p.pz);
-        rt[k] = zb + k < p.Z ? residual(p.vol_bar[(size_t)(zb + k) * plane + base], p.cnt[(size_t)(zb + k) * plane + base]) : 0.0f;
-        any |= rt[k] != 0.0f;
-    }
-    if (!any) return;
-    const float umax = (float)(p.U - 1), vmax = (float)(p.V - 1);
+// Adjoint of the backprojection: q_bar[view][iv][iu] += w[iu] rt x (bilinear
+// weights) over the voxels.
+//
+// A 16-byte vector reduction to global memory per sample is bound by its 28 to
+// 37 cycles an SM and warp request, whatever the lanes' addresses (measured; a
+// scalar one over 32 neighbouring pixels takes 7.6, and a load, an addition and
+// a store in shared memory 2.7).  So a warp sums the samples of a block of 8 x 8
+// columns and 32 slices in its own patch of the view, in shared memory, and
+// adds the patch to global memory once per view, about half a pixel a sample.
+// The lanes are 32 slices of one column: they fall on different rows, and where
+// consecutive slices are at least a row apart (checked per block and view) no
+// two lanes hold the same pixel, so plain additions serve, first to the
+// samples' upper rows, then to the lower ones; elsewhere shared-memory
+// reductions (4.1 cycles each).  Samples outside the patch (it holds kPatch
+// pixels; a sample on the last column has no right neighbour) go to global
+// memory by themselves.  What bounds it now is the shared memory: 20 wavefronts
+// a sample, eight of them bank conflicts (32 lanes spread over more than 32
+// rows).  A 64-view chunk of 256^3 from 512^2: 3.27 ms with the vector
+// reductions, 2.6 now, and the buffer of 16 bytes a pixel, its clearing and its
+// folding back to pixels are gone (0.11 ms).
+constexpr int kPatch = 1024, kAdjCols = 64, kAdjWarps = 4, kAdjBatch = 4;
+struct AdjWarp {
+    float patch[kPatch];
+    float rt[kAdjCols * 33];          // [column][slice], padded
+    float4 xy[kAdjCols];              // U, V, W at z = 0 and RN(1 / W) of the view
+};
+
+// rt times the bilinear weights at (u, v): lo on the upper row (left, right
+// pixel), hi on the lower one.
+__device__ __forceinline__ void adjoint_weights(float2 uv, float rt, float2& lo, float2& hi) {
+    const float2 magic = f2(kMagic, kMagic);
+    const float2 f = psub(uv, psub(padd_rm(uv, magic), magic));
+    const float b = rt * f.x;
+    const float2 ab = f2(rt - b, b);
+    hi = pmul(ab, f2(f.y, f.y));
+    lo = psub(ab, hi);
+}
+
+template <bool WZ, bool INSIDE>
+__device__ __forceinline__ void adjoint_views(const AdjParams& p, AdjWarp& m, int x0, int y0, int zb) {
+    const int lane = threadIdx.x & 31;
+    const unsigned umax_bits = __float_as_uint((float)(p.U - 1)), vmax_bits = __float_as_uint((float)(p.V - 1));
+    const float az = bp_axis(zb + lane, p.Z, p.pz);
+    // this lane's corner of the block
+    const float xc = bp_axis(lane & 1 ? min(x0 + 8, p.X) - 1 : x0, p.X, p.pxy);
+    const float yc = bp_axis(lane & 2 ? min(y0 + 8, p.Y) - 1 : y0, p.Y, p.pxy);
+    const float zc = bp_axis(lane & 4 ? min(zb + 32, p.Z) - 1 : zb, p.Z, p.pz);
+    const float2 magic = f2(kMagic, kMagic);
     const float4* P4 = reinterpret_cast<const float4*>(p.ptm + (size_t)p.v0 * 12);
-    float4* __restrict__ qb = p.qbar;
+    float* out = p.qbar;
 #pragma unroll 1
-    for (int n = 0; n < p.nv; ++n, P4 += 3, qb += p.q_frame) {
+    for (int n = 0; n < p.nv; ++n, P4 += 3, out += p.q_frame) {
         const float4 r0 = __ldg(P4), r1 = __ldg(P4 + 1), r2 = __ldg(P4 + 2);
-        const XYTerms xy = bp_xy_terms(ax, ay, r0, r1, r2);
-        const Recip rc = WZ ? Recip{0.0f, 0.0f} : bp_recip(xy.W);
+        const float2* __restrict__ tw = p.tw + (size_t)((p.v0 + n) % p.num_views) * p.U;
+        __syncwarp();   // the last view's columns and patch are done with
 #pragma unroll
-        for (int k = 0; k < ZPT; ++k) {
-            const float2 uv = bp_uv<false, WZ>(xy, rc, az[k], r0.z, r1.z, r2.z);
-            const bool in = (uv.x >= 0.0f) & (uv.x <= umax) & (uv.y >= 0.0f) & (uv.y <= vmax);
-            if (in && rt[k] != 0.0f) {
-                // floor by the 2^23 add rounded toward -inf (exact for 0 <= u, v < 2^23)
-                const float2 t = padd_rm(uv, f2(kMagic, kMagic));
-                const float2 f = psub(uv, psub(t, f2(kMagic, kMagic)));
-                const unsigned iu = __float_as_uint(t.x) - (unsigned)kMagicBits;
-                const unsigned iv = __float_as_uint(t.y) - (unsigned)kMagicBits;
-                const float a = rt[k] * (1.0f - f.x), b = rt[k] * f.x;
-                red_add_v4(qb + (size_t)iv * p.U + iu, make_float4(a * (1.0f - f.y), a * f.y, b * (1.0f - f.y), b * f.y));
+        for (int c = lane; c < kAdjCols; c += 32) {
+            const XYTerms t = bp_xy_terms(bp_axis(min(x0 + (c & 7), p.X - 1), p.X, p.pxy),
+                                          bp_axis(min(y0 + (c >> 3), p.Y - 1), p.Y, p.pxy), r0, r1, r2);
+            m.xy[c] = make_float4(t.U, t.V, t.W, WZ ? 0.0f : rcp_rn_nr(t.W));
+        }
+        // the patch: the block's corners in the view, a little around them
+        int c0 = 0, w = 0, row0 = 0, h = 0;
+        bool apart = false;
+        {
+            const float Vxy = fmaf(xc, r1.x, fmaf(yc, r1.y, r1.w)), Wxy = fmaf(xc, r2.x, fmaf(yc, r2.y, r2.w));
+            const float U = fmaf(zc, r0.z, fmaf(xc, r0.x, fmaf(yc, r0.y, r0.w)));
+            const float V = fmaf(zc, r1.z, Vxy), W = fmaf(zc, r2.z, Wxy);
+            const float u = __fdividef(U, W) + 0.5f, v = __fdividef(V, W) + 0.5f;
+            // dv/dz = (P6 W - P10 V) / W^2, its numerator the same in every slice
+            const float d = fmaf(r1.z, Wxy, -r2.z * Vxy);
+            float lo[4] = {u, v, W, d}, hi[4] = {u, v, W, d};
+#pragma unroll
+            for (int o = 1; o <= 4; o <<= 1)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    lo[i] = fminf(lo[i], __shfl_xor_sync(0xffffffffu, lo[i], o));
+                    hi[i] = fmaxf(hi[i], __shfl_xor_sync(0xffffffffu, hi[i], o));
+                }
+            const float um = (float)(p.U - 1), vm = (float)(p.V - 1);
+            // (comparisons false for NaN leave the patch empty)
+            if (lo[2] > 0.0f && hi[0] >= 0.0f && lo[0] <= um && hi[1] >= 0.0f && lo[1] <= vm) {
+                c0 = (int)fmaxf(lo[0] - 0.05f, 0.0f);
+                row0 = (int)fmaxf(lo[1] - 0.05f, 0.0f);
+                w = (int)fminf(hi[0] + 1.05f, um) - c0 + 1;
+                h = (int)fminf(hi[1] + 1.05f, vm) - row0 + 1;
+                const float dmin = lo[3] > 0.0f ? lo[3] : -hi[3];
+                apart = p.pz * dmin > 1.01f * hi[2] * hi[2];
             }
+        }
+        const int pitch = w | 1;   // odd: lanes a row apart use different banks
+        const int full = h;
+        h = min(h, kPatch / pitch);
+        const unsigned wlim = (unsigned)max(w - 1, 0), hlim = (unsigned)max(h - 1, 0);
+        // every sample of the block's voxels lies in the patch
+        const bool whole = INSIDE && w > 0 && h == full;
+        const float pf = (float)pitch;
+        // the patch's address less that of pixel (row0, c0) and of 2^23's bits
+        float* const base = m.patch - (row0 * pitch + c0);
+        const bool zin = zb + lane < p.Z;
+        __syncwarp();
+        if (whole && apart) {
+#pragma unroll 1
+            for (int cb = 0; cb < kAdjCols; cb += kAdjBatch) {
+                // the places and weights of kAdjBatch columns first, side by
+                // side: the additions below follow one another
+                float* s[kAdjBatch];
+                float2 lo[kAdjBatch], hi[kAdjBatch];
+#pragma unroll
+                for (int k = 0; k < kAdjBatch; ++k) {
+                    const float4 xw = m.xy[cb + k];
+                    const Recip rc{xw.w, WZ ? 0.0f : __fmul_rn(fmaf(-xw.z, xw.w, 1.0f), xw.w)};
+                    const float2 uv = bp_uv<false, WZ>(XYTerms{xw.x, xw.y, xw.z}, rc, az, r0.z, r1.z, r2.z);
+                    adjoint_weights(uv, m.rt[(cb + k) * 33 + lane], lo[k], hi[k]);
+                    const float2 t = padd_rm(uv, magic);
+                    s[k] = base + (__float_as_int(fmaf(__fsub_rn(t.y, kMagic), pf, t.x)) - kMagicBits);
+                }
+#pragma unroll
+                for (int k = 0; k < kAdjBatch; ++k) {
+                    if (zin) { s[k][0] += lo[k].x; s[k][1] += lo[k].y; }
+                    __syncwarp();
+                    if (zin) { s[k][pitch] += hi[k].x; s[k][pitch + 1] += hi[k].y; }
+                    __syncwarp();
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (int c = 0; c < kAdjCols; ++c) {
+                const float4 xw = m.xy[c];
+                const float rt = m.rt[c * 33 + lane];
+                const Recip rc{xw.w, WZ ? 0.0f : __fmul_rn(fmaf(-xw.z, xw.w, 1.0f), xw.w)};
+                float2 uv = bp_uv<false, WZ>(XYTerms{xw.x, xw.y, xw.z}, rc, az, r0.z, r1.z, r2.z);
+                const bool in = (rt != 0.0f) & (INSIDE || ((__float_as_uint(uv.x) <= umax_bits) & (__float_as_uint(uv.y) <= vmax_bits)));
+                uv = in ? uv : f2(0.0f, 0.0f);
+                float2 lo, hi;
+                adjoint_weights(uv, rt, lo, hi);
+                const float2 t = padd_rm(uv, magic);
+                const int iu = __float_as_int(t.x) - kMagicBits, iv = __float_as_int(t.y) - kMagicBits;
+                const bool inner = ((unsigned)(iu - c0) < wlim) & ((unsigned)(iv - row0) < hlim);
+                if (in & inner) {
+                    float* s = base + (iv * pitch + iu);
+                    atomicAdd(s, lo.x); atomicAdd(s + 1, lo.y);
+                    atomicAdd(s + pitch, hi.x); atomicAdd(s + pitch + 1, hi.y);
+                } else if (in) {   // pixels past the last row and column do not exist (their weight is 0)
+                    float* g = out + (size_t)iv * p.U + iu;
+                    const bool right = iu + 1 < p.U, down = iv + 1 < p.V;
+                    const float wl = tw[iu].x, wr = right ? tw[iu + 1].x : 0.0f;
+                    atomicAdd(g, wl * lo.x);
+                    if (right) atomicAdd(g + 1, wr * lo.y);
+                    if (down) atomicAdd(g + p.U, wl * hi.x);
+                    if (right && down) atomicAdd(g + p.U + 1, wr * hi.y);
+                }
+            }
+        }
+        __syncwarp();
+        // add the patch to the view, and clear it for the next one
+        const int dr = 32 / pitch, dc = 32 % pitch;
+        int row = lane / pitch, col = lane % pitch;
+        for (int i = lane; i < pitch * h; i += 32) {
+            const float v = m.patch[i];
+            if (v != 0.0f) {   // (true for NaN)
+                m.patch[i] = 0.0f;
+                atomicAdd(out + (size_t)(row0 + row) * p.U + c0 + col, v * tw[c0 + col].x);
+            }
+            row += dr;
+            col += dc;
+            if (col >= pitch) { col -= pitch; ++row; }
         }
     }
 }
 
-// Quad space -> detector pixels: p[r][c] appears in quads (r, c).x,
-// (r-1, c).y, (r, c-1).z, (r-1, c-1).w, each times the taper w[c].
-__global__ void __launch_bounds__(256) unpack_adjoint_kernel(const float4* __restrict__ qbar, long long q_frame,
-                                                             int rows, int U, const float2* __restrict__ tw,
-                                                             int view0, int num_views, float* __restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = blockIdx.y, f = blockIdx.z;
-    if (c >= U) return;
-    const float4* q = qbar + (size_t)f * q_frame;
-    float s = q[(size_t)r * U + c].x;
-    if (r > 0) s += q[(size_t)(r - 1) * U + c].y;
-    if (c > 0) s += q[(size_t)r * U + c - 1].z;
-    if (r > 0 && c > 0) s += q[(size_t)(r - 1) * U + c - 1].w;
-    const float w = tw[(size_t)((view0 + f) % num_views) * U + c].x;
-    out[(size_t)f * rows * U + (size_t)r * U + c] = w * s;
+template <bool WZ>
+__global__ void __launch_bounds__(32 * kAdjWarps, 4) bp_adjoint_kernel(AdjParams p) {
+    extern __shared__ AdjWarp adj_warps[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    AdjWarp& m = adj_warps[warp];
+    const int x0 = blockIdx.x * 16 + (warp & 1) * 8, y0 = blockIdx.y * 16 + (warp >> 1) * 8, zb = blockIdx.z * 32;
+    if (x0 >= p.X || y0 >= p.Y) return;   // (the warps do not wait for each other)
+    for (int i = lane; i < kPatch; i += 32) m.patch[i] = 0.0f;
+    const size_t plane = (size_t)p.X * p.Y;
+    bool any = false;
+    // 8 voxels in x by 4 slices to a load
+    const int x = x0 + (lane & 7);
+    for (int i = 0; i < 64; ++i) {
+        const int y = y0 + (i & 7), z = (i >> 3) * 4 + (lane >> 3);
+        float r = 0.0f;
+        if (x < p.X && y < p.Y && zb + z < p.Z) {
+            const size_t at = (size_t)(zb + z) * plane + (size_t)y * p.X + x;
+            r = residual(p.vol_bar[at], p.cnt[at]);
+        }
+        m.rt[((i & 7) * 8 + (lane & 7)) * 33 + z] = r;
+        any |= r != 0.0f;
+    }
+    if (!__any_sync(0xffffffffu, any)) return;
+    bool ok = true;
+    const VoxelBox box(bp_axis(x0, p.X, p.pxy), bp_axis(min(x0 + 8, p.X) - 1, p.X, p.pxy), bp_axis(y0, p.Y, p.pxy),
+                       bp_axis(min(y0 + 8, p.Y) - 1, p.Y, p.pxy), bp_axis(zb, p.Z, p.pz), bp_axis(zb + 31, p.Z, p.pz));
+    for (int n = lane; n < p.nv; n += 32) ok = ok && box_inside(box, p.ptm + (size_t)(p.v0 + n) * 12, p.U, p.V);
+    if (__all_sync(0xffffffffu, ok))
+        adjoint_views<WZ, true>(p, m, x0, y0, zb);
+    else
+        adjoint_views<WZ, false>(p, m, x0, y0, zb);
 }
 
 // Geometry gradient: per (CTA, view) partial sums of the 6 components.
@@ -308,28 +445,20 @@ __global__ void pad_rows_kernel(const float* __restrict__ src, int w, float* __r
     for (int i = threadIdx.x; i < pitch; i += blockDim.x) dst[m * pitch + i] = i < w ? src[m * w + i] : 0.0f;
 }
 
-template <int ZPT>
-dim3 bp_grid(const AdjParams& p) {
-    return dim3((p.X + 31) / 32, (p.Y + 7) / 8, (p.Z + ZPT - 1) / ZPT);
-}
-
 }  // namespace
 
 cudaError_t launch_bp_adjoint(const AdjParams& p, bool wz, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(p.qbar, 0, sizeof(float4) * (size_t)p.nv * p.q_frame, s);
+    constexpr int smem = kAdjWarps * (int)sizeof(AdjWarp);
+    // (per call: the attribute belongs to the current device)
+    cudaError_t e = wz ? cudaFuncSetAttribute(bp_adjoint_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
+                       : cudaFuncSetAttribute(bp_adjoint_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p.qbar, 0, sizeof(float) * (size_t)p.nv * p.q_frame, s);
     if (e != cudaSuccess) return e;
-    const dim3 g = bp_grid<kAdjZpt>(p);
+    const dim3 grid((p.X + 15) / 16, (p.Y + 15) / 16, (p.Z + 31) / 32);
     if (wz)
-        bp_adjoint_kernel<kAdjZpt, true><<<g, dim3(32, 8), 0, s>>>(p);
+        bp_adjoint_kernel<true><<<grid, 32 * kAdjWarps, smem, s>>>(p);
     else
-        bp_adjoint_kernel<kAdjZpt, false><<<g, dim3(32, 8), 0, s>>>(p);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_unpack_adjoint(const float4* qbar, long long q_frame, int nv, int rows, int U, const float2* tw,
-                                  int view0, int num_views, float* out, cudaStream_t s) {
-    dim3 grid((U + 255) / 256, rows, nv);
-    unpack_adjoint_kernel<<<grid, 256, 0, s>>>(qbar, q_frame, rows, U, tw, view0, num_views, out);
+        bp_adjoint_kernel<false><<<grid, 32 * kAdjWarps, smem, s>>>(p);
     return cudaGetLastError();
 }
 

@@ -297,6 +297,18 @@ int bp_zpt(const jfdk_ctx* c) {
     return tiles >= 8LL * 5 * c->sms ? 16 : 8;
 }
 
+// The depth a launch over nz slices runs with: in the FP32 form, whose volume
+// does not depend on it, 4 instead of the default 8 where 8-slice tiles fill at
+// most half of a wave (6 CTAs per SM): 64^3 from 180 views (256 tiles) 280 us
+// against 350; at 864 tiles, nearly a full wave, 708 against 617.
+int launch_zpt(const jfdk_ctx* c, int nz) {
+    const int zpt = bp_zpt(c);
+    if (mixed(c) || c->opt_bp_zpt) return zpt;
+    const long long tiles = (long long)((c->X + kBPTileX - 1) / kBPTileX) * ((c->Y + kBPTileY - 1) / kBPTileY) *
+                            ((nz + zpt - 1) / zpt);
+    return tiles <= 3LL * c->sms ? 4 : zpt;
+}
+
 // CTA width in x: the option, else 4 (4 x 32 threads).
 int bp_tile(const jfdk_ctx* c) { return c->opt_bp_tile ? c->opt_bp_tile : kBPTileX; }
 
@@ -382,7 +394,7 @@ jfdk_status run_bp_on(jfdk_ctx* c, BPParams b, bool finalize, cudaStream_t s) {
         JFDK_LAUNCH(c, launch_bp_mixed(b, finalize, geometry(c), bp_zpt(c), bp_tile(c), s), "backprojection");
         return JFDK_OK;
     }
-    JFDK_LAUNCH(c, launch_bp(b, finalize, c->opt_bp_exact != 0, geometry(c), bp_zpt(c), bp_tile(c), s),
+    JFDK_LAUNCH(c, launch_bp(b, finalize, c->opt_bp_exact != 0, geometry(c), launch_zpt(c, b.z_end - b.z_begin), bp_tile(c), s),
                 "backprojection");
     return JFDK_OK;
 }
@@ -556,7 +568,7 @@ void jfdk_destroy(jfdk_ctx* c) {
     dev_free(c, c->d_plain);
     dev_free(c, c->d_q4); dev_free(c, c->d_qscale); dev_free(c, c->d_absmax);
     dev_free(c, c->d_sum); dev_free(c, c->d_cnt); dev_free(c, c->d_raw_stage); dev_free(c, c->d_hu_stage);
-    dev_free(c, c->d_Tt); dev_free(c, c->d_qadj); dev_free(c, c->d_partial);
+    dev_free(c, c->d_Tt); dev_free(c, c->d_partial);
     dev_free(c, c->d_dptm);
     dev_free(c, c->d_wvol);
     for (auto& e : c->ev)
@@ -1228,18 +1240,9 @@ jfdk_status jfdk_bp_adjoint(jfdk_ctx* c, const float* d_vol_bar, int v0, int nv,
         return fail(c, JFDK_ERR_INVALID, "bp_adjoint: bad argument");
     jfdk_status st = deriv_check(c, "bp_adjoint");
     if (st || nv == 0) return st;
-    if (c->qadj_views < nv) {
-        dev_free(c, c->d_qadj);
-        c->qadj_views = 0;
-        if ((st = dev_alloc(c, &c->d_qadj, (size_t)nv * frame_px(c), "the quad-space adjoint"))) return st;
-        c->qadj_views = nv;
-    }
     AdjParams a = adj_params(c, d_vol_bar, v0, nv);
-    a.qbar = c->d_qadj;
+    a.qbar = d_q_bar;
     JFDK_LAUNCH(c, launch_bp_adjoint(a, c->w_depends_on_z, c->stream), "backprojection adjoint");
-    JFDK_LAUNCH(c, launch_unpack_adjoint(c->d_qadj, frame_px(c), nv, c->rows, c->out_w, c->d_tw, v0, c->nviews,
-                                         d_q_bar, c->stream),
-                "backprojection adjoint (unpack)");
     return JFDK_OK;
 }
 

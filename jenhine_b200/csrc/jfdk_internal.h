@@ -259,7 +259,7 @@ struct AdjParams {
     float pxy, pz;
     const float* vol_bar;    // [Z][Y][X] dL / dvol
     const float* cnt;        // [Z][Y][X] the forward's weights: rt = vol_bar / cnt
-    float4* qbar;            // adjoint out: quad space [nv][V][U]
+    float* qbar;             // adjoint out: detector pixels [nv][V][U]
     long long q_frame;       // V * U
     const float4* q4;        // gradient: the forward's tapered quads [nv][V][U]
     const float2* tw;        // [views][U] taper pairs (w[c], RN(w[c+1] - w[c]))
@@ -269,8 +269,6 @@ struct AdjParams {
     int sms;
 };
 cudaError_t launch_bp_adjoint(const AdjParams& p, bool w_depends_on_z, cudaStream_t s);
-cudaError_t launch_unpack_adjoint(const float4* qbar, long long q_frame, int nv, int rows, int U, const float2* tw,
-                                  int view0, int num_views, float* out, cudaStream_t s);
 size_t geometry_gradient_ctas(const AdjParams& p);
 cudaError_t launch_geometry_gradient(const AdjParams& p, bool w_depends_on_z, double* grad, cudaStream_t s);
 cudaError_t launch_pad_rows(const float* src, size_t rows, int w, float* dst, int pitch, cudaStream_t s);
@@ -347,7 +345,6 @@ struct jfdk_ctx {
     float* d_hu_stage = nullptr; size_t hu_stage_bytes = 0;
     bool bp_has_views = false;
     // derivatives (allocated on demand)
-    float4* d_qadj = nullptr; int qadj_views = 0;    // quad-space adjoint
     float* d_partial = nullptr; size_t partial_n = 0;
     float* d_dptm = nullptr; int dptm_views = 0;
 
