@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 4) bp_adjoint_kernel(AdjParams
     bool ok = true;
     const VoxelBox box(bp_axis(x0, p.X, p.pxy), bp_axis(min(x0 + 8, p.X) - 1, p.X, p.pxy), bp_axis(y0, p.Y, p.pxy),
                        bp_axis(min(y0 + 8, p.Y) - 1, p.Y, p.pxy), bp_axis(zb, p.Z, p.pz), bp_axis(zb + 31, p.Z, p.pz));
-    for (int n = lane; n < p.nv; n += 32) ok = ok && box_inside(box, p.ptm + (size_t)(p.v0 + n) * 12, p.U, p.V);
+    for (int n = lane; n < p.nv; n += 32) ok = ok && box_place(box, p.ptm + (size_t)(p.v0 + n) * 12, p.U, p.V) == kBoxInside;
     if (__all_sync(0xffffffffu, ok))
         adjoint_views<WZ, true>(p, m, x0, y0, zb);
     else
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kGradThreads, 4) geometry_gradient_kernel(AdjP
     const VoxelBox box(bp_axis(xb, p.X, p.pxy), bp_axis(min(xb + 8 * J, p.X) - 1, p.X, p.pxy), bp_axis(yb, p.Y, p.pxy),
                        bp_axis(min(yb + kGradRows, p.Y) - 1, p.Y, p.pxy), bp_axis(zb, p.Z, p.pz),
                        bp_axis(zb + ZPT - 1, p.Z, p.pz));
-    for (int n = tid; n < p.nv; n += kGradThreads) ok = ok && box_inside(box, p.ptm + (size_t)(p.v0 + n) * 12, p.U, p.V);
+    for (int n = tid; n < p.nv; n += kGradThreads) ok = ok && box_place(box, p.ptm + (size_t)(p.v0 + n) * 12, p.U, p.V) == kBoxInside;
     // threads past the volume's edge walk its last row and column with rt = 0
     const int yc = min(y, p.Y - 1);
     if (__syncthreads_and(ok))

@@ -206,18 +206,23 @@ struct VoxelBox {
           my(fmaxf(fabsf(y0), fabsf(y1))), mz(fmaxf(fabsf(z0), fabsf(z1))) {}
 };
 
-// Whether every voxel of the box samples the view of matrix P inside a U x V
-// detector, in front of the source.  0 <= u <= U - 1, 0 <= v <= V - 1 and W > 0
-// are linear in the voxel's place once multiplied by W, so the least value over
-// the box is the one at its centre minus the coefficients' moduli times the
-// half extents: five such values.  The margin, 2^-16 of the sum of the terms'
-// moduli, is far above what the rounded coordinates can be off (a few 2^-24 of
-// that sum, 16 steps of it in the mixed form), so no sample of a box that
-// passes would be turned down by the range test.
-__device__ __forceinline__ bool box_inside(const VoxelBox& b, const float* P, int U, int V) {
+// Where the voxels of the box sample the view of matrix P on a U x V detector:
+// kBoxInside, every one at 0 <= u <= U - 1, 0 <= v <= V - 1 in front of the
+// source (W > 0); kBoxOutside, none; kBoxAcross, not known.  The conditions
+// are linear in the voxel's place once multiplied by W, so the least and the
+// largest value over the box are the one at its centre minus and plus the
+// coefficients' moduli times the half extents: five linear forms.  The margin,
+// 2^-16 of the sum of the terms' moduli, is far above what the rounded
+// coordinates can be off (a few 2^-24 of that sum, 16 steps of it in the mixed
+// form), so the range test would take every sample of a box inside and none of
+// a box outside.
+enum BoxPlace { kBoxAcross = 0, kBoxInside = 1, kBoxOutside = 2 };
+
+__device__ __forceinline__ BoxPlace box_place(const VoxelBox& b, const float* P, int U, int V) {
     const float4* P4 = reinterpret_cast<const float4*>(P);
     const float4 r0 = __ldg(P4), r1 = __ldg(P4 + 1), r2 = __ldg(P4 + 2);
-    // least value of k r + l r2 (rows of the matrix) over the box, against the margin
+    bool inside = true, outside = false;
+    // k r + l r2 (rows of the matrix) over the box, against the margin
     auto clear = [&](const float4& r, float k, float l, float lim) {
         const float kx = fmaf(k, r.x, l * r2.x), ky = fmaf(k, r.y, l * r2.y), kz = fmaf(k, r.z, l * r2.z);
         const float f = fmaf(kx, b.cx, fmaf(ky, b.cy, fmaf(kz, b.cz, fmaf(k, r.w, l * r2.w))));
@@ -225,11 +230,19 @@ __device__ __forceinline__ bool box_inside(const VoxelBox& b, const float* P, in
         const float m = fmaf(fmaf(lim, fabsf(r2.x), fabsf(r.x)), b.mx,
                              fmaf(fmaf(lim, fabsf(r2.y), fabsf(r.y)), b.my,
                                   fmaf(fmaf(lim, fabsf(r2.z), fabsf(r.z)), b.mz, fmaf(lim, fabsf(r2.w), fabsf(r.w)))));
-        return f - h > 0x1p-16f * m;   // false for NaN
+        inside = inside && f - h > 0x1p-16f * m;     // both false for NaN
+        outside = outside || f + h < -0x1p-16f * m;
     };
     const float ul = (float)U, vl = (float)V;
-    return clear(r2, 1.0f, 0.0f, 1.0f) && clear(r0, 1.0f, 0.5f, ul) && clear(r0, -1.0f, ul - 1.5f, ul) &&
-           clear(r1, 1.0f, 0.5f, vl) && clear(r1, -1.0f, vl - 1.5f, vl);
+    clear(r2, 1.0f, 0.0f, 1.0f);
+    // u and v have the signs of these forms in front of the source only
+    const bool front = inside;
+    outside = false;
+    clear(r0, 1.0f, 0.5f, ul);
+    clear(r0, -1.0f, ul - 1.5f, ul);
+    clear(r1, 1.0f, 0.5f, vl);
+    clear(r1, -1.0f, vl - 1.5f, vl);
+    return inside ? kBoxInside : front && outside ? kBoxOutside : kBoxAcross;
 }
 
 }  // namespace
