@@ -1,7 +1,7 @@
 // bp_body.cuh -- voxel-driven cone-beam backprojection with fused normalisation and
 // CT numbers (sm_100a): the bodies of the kernels, which bp_fast.cu, bp_exact.cu,
-// bp_weights.cu, bp_mixed.cu and bp_batch.cu instantiate (one file each, so
-// that they compile side by side).
+// bp_weights.cu, bp_mixed.cu, bp_wide.cu and bp_batch.cuh instantiate (one file
+// each, so that they compile side by side).
 //
 // Semantics follow the reference's CPU backprojector, BPCore
 // (BPAgent/BPCore.cpp:115-220):
@@ -32,10 +32,8 @@
 // stores the volume once and never reads it.
 //
 // Arithmetic.  U, V are formed exactly as BPCore rounds them.  The quotients
-// are computed as a pair (packed f32x2) from one correctly
-// rounded reciprocal r = RN(1/W) and Markstein's correction q = RN(q0 + RN(U -
-// W q0) r), q0 = RN(U r), which yields RN(U / W); when P[10] == 0 for every
-// view W does not depend on z (BPCore adds z*0) and r is computed once per
+// come from one reciprocal (bp_quotient2); when P[10] == 0 for every view W does
+// not depend on z (BPCore adds z*0) and the reciprocal is computed once per
 // (x, y, view).  EXACT additionally rounds the lerps step by step like
 // BPCore (every product and sum separately) instead of fusing them.
 #pragma once
@@ -199,7 +197,7 @@ __device__ __forceinline__ float taper_lerp(float2 w, float fx) {
 // data pipe for as long (6 wavefronts a request: four, and one for each second
 // quarter-warp whose records cross a 128-byte line).  c2, 1.18e11 samples:
 // 127.9 ms with range tests, 64-bit addresses, Markstein's quotient and one
-// view at a time, 104.6 now (33.5 cycles a sample and scheduler).  At kGeoIdeal
+// view at a time, 102.8 now (33 cycles a sample and scheduler).  At kGeoIdeal
 // u is the view's and V, v and the rest are formed for two slices at a time, 14
 // cycles of the FMA pipe a sample.
 // Measured and left out: floor on the conversion pipe (0.9 ms of 114 faster,

@@ -1,4 +1,4 @@
-// bp_common.cuh -- device helpers shared by the backprojector (bp.cu) and its
+// bp_common.cuh -- device helpers shared by the backprojector (bp_body.cuh) and its
 // adjoint / geometry gradient (adjoint.cu): packed f32x2 arithmetic, the
 // floor trick, CT numbers, and the sample coordinates of the FP32 form, so the
 // adjoint sees exactly the forward's sample points and in-range decisions.
