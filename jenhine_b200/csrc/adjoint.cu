@@ -70,7 +70,7 @@ __device__ __forceinline__ void adjoint_weights(float2 uv, float rt, float2& lo,
 }
 
 template <bool WZ, bool INSIDE>
-__device__ __forceinline__ void adjoint_views(const AdjParams& p, AdjWarp& m, int x0, int y0, int zb) {
+__device__ __forceinline__ void adjoint_views(const AdjParams& p, AdjWarp& m, const VoxelBox& box, int x0, int y0, int zb) {
     const int lane = threadIdx.x & 31;
     const unsigned umax_bits = __float_as_uint((float)(p.U - 1)), vmax_bits = __float_as_uint((float)(p.V - 1));
     const float az = bp_axis(zb + lane, p.Z, p.pz);
@@ -95,6 +95,7 @@ __device__ __forceinline__ void adjoint_views(const AdjParams& p, AdjWarp& m, in
         // the patch: the block's corners in the view, a little around them
         int c0 = 0, w = 0, row0 = 0, h = 0;
         bool apart = false;
+        float wmin = 0.0f;
         {
             const float Vxy = fmaf(xc, r1.x, fmaf(yc, r1.y, r1.w)), Wxy = fmaf(xc, r2.x, fmaf(yc, r2.y, r2.w));
             const float U = fmaf(zc, r0.z, fmaf(xc, r0.x, fmaf(yc, r0.y, r0.w)));
@@ -119,17 +120,27 @@ __device__ __forceinline__ void adjoint_views(const AdjParams& p, AdjWarp& m, in
                 h = (int)fminf(hi[1] + 1.05f, vm) - row0 + 1;
                 const float dmin = lo[3] > 0.0f ? lo[3] : -hi[3];
                 apart = p.pz * dmin > 1.01f * hi[2] * hi[2];
+                wmin = lo[2];
             }
         }
         const int pitch = w | 1;   // odd: lanes a row apart use different banks
         const int full = h;
         h = min(h, kPatch / pitch);
         const unsigned wlim = (unsigned)max(w - 1, 0), hlim = (unsigned)max(h - 1, 0);
-        // every sample of the block's voxels lies in the patch
-        const bool whole = INSIDE && w > 0 && h == full;
+        // Every sample of the block's voxels lies in the patch, and consecutive
+        // slices' rows differ: the rounded places are within 2^-22 of the sum of
+        // the terms' moduli (over W), which has to be far below the 0.05 pixels
+        // around the corners and the hundredth of a row above one; and the
+        // patch's index below is exact in a float.
+        const float lim = (float)(p.U + p.V);
+        const float moduli = fmaf(box.mx, fabsf(r0.x) + fabsf(r1.x) + lim * fabsf(r2.x),
+                                  fmaf(box.my, fabsf(r0.y) + fabsf(r1.y) + lim * fabsf(r2.y),
+                                       fmaf(box.mz, fabsf(r0.z) + fabsf(r1.z) + lim * fabsf(r2.z),
+                                            fabsf(r0.w) + fabsf(r1.w) + lim * fabsf(r2.w))));
+        const bool whole = INSIDE && w > 0 && h == full && moduli * 0x1p-22f < 0.004f * wmin &&
+                           (long long)(row0 + h) * pitch + c0 + w < (1LL << 23);
         const float pf = (float)pitch;
-        // the patch's address less that of pixel (row0, c0) and of 2^23's bits
-        float* const base = m.patch - (row0 * pitch + c0);
+        const int first = row0 * pitch + c0;
         const bool zin = zb + lane < p.Z;
         __syncwarp();
         if (whole && apart) {
@@ -146,7 +157,9 @@ __device__ __forceinline__ void adjoint_views(const AdjParams& p, AdjWarp& m, in
                     const float2 uv = bp_uv<false, WZ>(XYTerms{xw.x, xw.y, xw.z}, rc, az, r0.z, r1.z, r2.z);
                     adjoint_weights(uv, m.rt[(cb + k) * 33 + lane], lo[k], hi[k]);
                     const float2 t = padd_rm(uv, magic);
-                    s[k] = base + (__float_as_int(fmaf(__fsub_rn(t.y, kMagic), pf, t.x)) - kMagicBits);
+                    const int at = __float_as_int(fmaf(__fsub_rn(t.y, kMagic), pf, t.x)) - kMagicBits - first;
+                    // (a lane past the last slice has no place in the patch)
+                    s[k] = m.patch + (zin ? at : 0);
                 }
 #pragma unroll
                 for (int k = 0; k < kAdjBatch; ++k) {
@@ -171,7 +184,7 @@ __device__ __forceinline__ void adjoint_views(const AdjParams& p, AdjWarp& m, in
                 const int iu = __float_as_int(t.x) - kMagicBits, iv = __float_as_int(t.y) - kMagicBits;
                 const bool inner = ((unsigned)(iu - c0) < wlim) & ((unsigned)(iv - row0) < hlim);
                 if (in & inner) {
-                    float* s = base + (iv * pitch + iu);
+                    float* s = m.patch + (iv * pitch + iu - first);
                     atomicAdd(s, lo.x); atomicAdd(s + 1, lo.y);
                     atomicAdd(s + pitch, hi.x); atomicAdd(s + pitch + 1, hi.y);
                 } else if (in) {   // pixels past the last row and column do not exist (their weight is 0)
@@ -230,9 +243,9 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 4) bp_adjoint_kernel(AdjParams
                        bp_axis(min(y0 + 8, p.Y) - 1, p.Y, p.pxy), bp_axis(zb, p.Z, p.pz), bp_axis(zb + 31, p.Z, p.pz));
     for (int n = lane; n < p.nv; n += 32) ok = ok && box_place(box, p.ptm + (size_t)(p.v0 + n) * 12, p.U, p.V) == kBoxInside;
     if (__all_sync(0xffffffffu, ok))
-        adjoint_views<WZ, true>(p, m, x0, y0, zb);
+        adjoint_views<WZ, true>(p, m, box, x0, y0, zb);
     else
-        adjoint_views<WZ, false>(p, m, x0, y0, zb);
+        adjoint_views<WZ, false>(p, m, box, x0, y0, zb);
 }
 
 // Geometry gradient: per (CTA, view) partial sums of the 6 components.
