@@ -49,7 +49,7 @@ constexpr int kAdjZpt = 8;
 // memory by themselves.  What bounds it now is the shared memory: 20 wavefronts
 // a sample, eight of them bank conflicts (32 lanes spread over more than 32
 // rows).  A 64-view chunk of 256^3 from 512^2: 3.27 ms with the vector
-// reductions, 2.6 now, and the buffer of 16 bytes a pixel, its clearing and its
+// reductions, 2.7 now, and the buffer of 16 bytes a pixel, its clearing and its
 // folding back to pixels are gone (0.11 ms).
 constexpr int kPatch = 1024, kAdjCols = 64, kAdjWarps = 4, kAdjBatch = 4;
 struct AdjWarp {
