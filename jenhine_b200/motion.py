@@ -47,8 +47,14 @@ def _rigid_all(theta: np.ndarray, derivatives: bool = True):
 
 
 def rigid(theta) -> tuple[np.ndarray, np.ndarray]:
-    """M(theta) (4 x 4) and dM/dtheta_j (6 x 4 x 4), FP64."""
-    M, dM = _rigid_all(np.asarray(theta, np.float64)[:6])
+    """M(theta) (4 x 4) and dM/dtheta_j (6 x 4 x 4), FP64, of one motion (what
+    follows its six parameters is not read)."""
+    t = np.asarray(theta, np.float64)
+    if t.ndim == 0 or len(t) < 6:
+        raise IndexError(f"a motion has six parameters, got shape {t.shape}")
+    if t.ndim != 1:
+        raise ValueError(f"rigid takes one motion, got shape {t.shape}")
+    M, dM = _rigid_all(t[:6])
     return M[0], dM[0]
 
 
@@ -56,6 +62,8 @@ def _views(P0, theta):
     """P0 (n, 3, 4) and the motions of its views (a theta of more views is cut)."""
     P0 = np.asarray(P0, np.float64).reshape(-1, 3, 4)
     th = np.asarray(theta, np.float64).reshape(-1, 6)
+    if not len(P0):
+        raise ValueError("no projection matrices")
     if len(th) < len(P0):
         raise IndexError(f"{len(th)} motions for {len(P0)} views")
     return P0, th[:len(P0)]
