@@ -59,14 +59,16 @@ struct AdjWarp {
 };
 
 // rt times the bilinear weights at (u, v): lo on the upper row (left, right
-// pixel), hi on the lower one.
+// pixel), hi on the lower one.  Products of rt with each side's own weight, so
+// that a small one is as exact as a large one (1 - f is exact) and an infinite
+// rt gives infinities.
 __device__ __forceinline__ void adjoint_weights(float2 uv, float rt, float2& lo, float2& hi) {
     const float2 magic = f2(kMagic, kMagic);
     const float2 f = psub(uv, psub(padd_rm(uv, magic), magic));
-    const float b = rt * f.x;
-    const float2 ab = f2(rt - b, b);
+    const float2 g = psub(f2(1.0f, 1.0f), f);
+    const float2 ab = pmul(f2(rt, rt), f2(g.x, f.x));
     hi = pmul(ab, f2(f.y, f.y));
-    lo = psub(ab, hi);
+    lo = pmul(ab, f2(g.y, g.y));
 }
 
 template <bool WZ, bool INSIDE>
