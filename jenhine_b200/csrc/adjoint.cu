@@ -241,8 +241,10 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 4) bp_adjoint_kernel(AdjParams
     }
     if (!__any_sync(0xffffffffu, any)) return;
     bool ok = true;
+    // (lanes past the last slice add nothing: thin volumes are inside too)
     const VoxelBox box(bp_axis(x0, p.X, p.pxy), bp_axis(min(x0 + 8, p.X) - 1, p.X, p.pxy), bp_axis(y0, p.Y, p.pxy),
-                       bp_axis(min(y0 + 8, p.Y) - 1, p.Y, p.pxy), bp_axis(zb, p.Z, p.pz), bp_axis(zb + 31, p.Z, p.pz));
+                       bp_axis(min(y0 + 8, p.Y) - 1, p.Y, p.pxy), bp_axis(zb, p.Z, p.pz),
+                       bp_axis(min(zb + 32, p.Z) - 1, p.Z, p.pz));
     for (int n = lane; n < p.nv; n += 32) ok = ok && box_place(box, p.ptm + (size_t)(p.v0 + n) * 12, p.U, p.V) == kBoxInside;
     if (__all_sync(0xffffffffu, ok))
         adjoint_views<WZ, true>(p, m, box, x0, y0, zb);
