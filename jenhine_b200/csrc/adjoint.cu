@@ -3,7 +3,7 @@
 //   * the adjoint of the backprojector, vol = S q / C: with the weights C
 //     (the backprojected taper) fixed, q_bar = S^T (vol_bar / C) -- for every
 //     voxel and view the transposed bilinear weights of its sample point, summed
-//     in patches of the view in shared memory and multiplied by the taper;
+//     per pixel and multiplied by the taper;
 //   * the adjoint of the ramp filter, y = T (w o x) + c e(x) with
 //     e(x) = (x0 + x1 + x2) / 3 (or the last three for a mirrored filter):
 //     x_bar = w o (T^T y_bar) + (c . y_bar) / 3 on the edge samples;
@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 
 #include "bp_common.cuh"
@@ -31,33 +32,6 @@ __device__ __forceinline__ float residual(float vol_bar, float cnt) { return cnt
 
 constexpr int kAdjZpt = 8;
 
-// Adjoint of the backprojection: q_bar[view][iv][iu] += w[iu] rt x (bilinear
-// weights) over the voxels.
-//
-// A 16-byte vector reduction to global memory per sample is bound by its 28 to
-// 37 cycles an SM and warp request, whatever the lanes' addresses (measured; a
-// scalar one over 32 neighbouring pixels takes 7.6, and a load, an addition and
-// a store in shared memory 2.7).  So a warp sums the samples of a block of 8 x 8
-// columns and 32 slices in its own patch of the view, in shared memory, and
-// adds the patch to global memory once per view, about half a pixel a sample.
-// The lanes are 32 slices of one column: they fall on different rows, and where
-// consecutive slices are at least a row apart (checked per block and view) no
-// two lanes hold the same pixel, so plain additions serve, first to the
-// samples' upper rows, then to the lower ones; elsewhere shared-memory
-// reductions (4.1 cycles each).  Samples outside the patch (it holds kPatch
-// pixels; a sample on the last column has no right neighbour) go to global
-// memory by themselves.  What bounds it now is the shared memory: 20 wavefronts
-// a sample, eight of them bank conflicts (32 lanes spread over more than 32
-// rows).  A 64-view chunk of 256^3 from 512^2: 3.27 ms with the vector
-// reductions, 2.7 now, and the buffer of 16 bytes a pixel, its clearing and its
-// folding back to pixels are gone (0.11 ms).
-constexpr int kPatch = 1024, kAdjCols = 64, kAdjWarps = 4, kAdjBatch = 4;
-struct AdjWarp {
-    float patch[kPatch];
-    float rt[kAdjCols * 33];          // [column][slice], padded
-    float4 xy[kAdjCols];              // U, V, W at z = 0 and RN(1 / W) of the view
-};
-
 // rt times the bilinear weights at (u, v): lo on the upper row (left, right
 // pixel), hi on the lower one.  Products of rt with each side's own weight, so
 // that a small one is as exact as a large one (1 - f is exact) and an infinite
@@ -70,6 +44,101 @@ __device__ __forceinline__ void adjoint_weights(float2 uv, float rt, float2& lo,
     hi = pmul(ab, f2(f.y, f.y));
     lo = pmul(ab, f2(g.y, g.y));
 }
+
+// Adjoint of the backprojection, q_bar[view][iv][iu] += w[iu] rt x (bilinear
+// weights) over the voxels, in one of two ways (adjoint_by_patches chooses).
+//
+// By "quad space", the way of any scan and size: the forward's footprint records,
+// one 16-byte vector reduction per sample, folded back to pixels and multiplied
+// by the taper afterwards (unpack_adjoint_kernel).  A reduction takes 28 to 37
+// cycles an SM and warp request, whatever the lanes' addresses, which is what
+// bounds it; a thread per column and eight slices fills the GPU early.
+__device__ __forceinline__ void red_add_v4(float4* p, float4 v) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+
+template <bool WZ>
+__global__ void __launch_bounds__(256) bp_adjoint_quads_kernel(AdjParams p) {
+    constexpr int ZPT = kAdjZpt;
+    const int x = blockIdx.x * 32 + threadIdx.x;
+    const int y = blockIdx.y * 8 + threadIdx.y;
+    const int zb = blockIdx.z * ZPT;
+    if (x >= p.X || y >= p.Y) return;
+    const float ax = bp_axis(x, p.X, p.pxy), ay = bp_axis(y, p.Y, p.pxy);
+    const size_t plane = (size_t)p.X * p.Y, base = (size_t)y * p.X + x;
+    float az[ZPT], rt[ZPT];
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < ZPT; ++k) {
+        const size_t at = (size_t)(zb + k) * plane + base;
+        az[k] = bp_axis(zb + k, p.Z, p.pz);
+        rt[k] = zb + k < p.Z ? residual(p.vol_bar[at], p.cnt[at]) : 0.0f;
+        any |= rt[k] != 0.0f;
+    }
+    if (!any) return;
+    const unsigned umax_bits = __float_as_uint((float)(p.U - 1)), vmax_bits = __float_as_uint((float)(p.V - 1));
+    const float4* P4 = reinterpret_cast<const float4*>(p.ptm + (size_t)p.v0 * 12);
+    float4* __restrict__ qb = p.quads;
+#pragma unroll 1
+    for (int n = 0; n < p.nv; ++n, P4 += 3, qb += p.q_frame) {
+        const float4 r0 = __ldg(P4), r1 = __ldg(P4 + 1), r2 = __ldg(P4 + 2);
+        const XYTerms xy = bp_xy_terms(ax, ay, r0, r1, r2);
+        const Recip rc = WZ ? Recip{0.0f, 0.0f} : bp_recip(xy.W);
+#pragma unroll
+        for (int k = 0; k < ZPT; ++k) {
+            const float2 uv = bp_uv<false, WZ>(xy, rc, az[k], r0.z, r1.z, r2.z);
+            if ((__float_as_uint(uv.x) <= umax_bits) & (__float_as_uint(uv.y) <= vmax_bits) & (rt[k] != 0.0f)) {
+                float2 lo, hi;
+                adjoint_weights(uv, rt[k], lo, hi);
+                const float2 t = padd_rm(uv, f2(kMagic, kMagic));
+                const unsigned iu = __float_as_uint(t.x) - (unsigned)kMagicBits;
+                const unsigned iv = __float_as_uint(t.y) - (unsigned)kMagicBits;
+                red_add_v4(qb + (size_t)iv * p.U + iu, make_float4(lo.x, hi.x, lo.y, hi.y));
+            }
+        }
+    }
+}
+
+// Quad space -> detector pixels: p[r][c] appears in quads (r, c).x,
+// (r-1, c).y, (r, c-1).z, (r-1, c-1).w, each times the taper w[c].
+__global__ void __launch_bounds__(256) unpack_adjoint_kernel(AdjParams p) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= p.U) return;
+    for (int f = blockIdx.z; f < p.nv; f += gridDim.z) {
+        const float4* q = p.quads + (size_t)f * p.q_frame + c;
+        float* out = p.qbar + (size_t)f * p.q_frame + c;
+        const float w = p.tw[(size_t)((p.v0 + f) % p.num_views) * p.U + c].x;
+        for (int r = blockIdx.y; r < p.V; r += gridDim.y) {
+            const float4* at = q + (size_t)r * p.U;
+            float s = at->x;
+            if (r > 0) s += (at - p.U)->y;
+            if (c > 0) s += (at - 1)->z;
+            if (r > 0 && c > 0) s += (at - p.U - 1)->w;
+            out[(size_t)r * p.U] = w * s;
+        }
+    }
+}
+
+// By patches: a warp sums the samples of a block of 8 x 8 columns and 32 slices
+// in its own patch of the view, in shared memory (a load, an addition and a
+// store there take 2.7 cycles a request, a scalar reduction to global memory over
+// 32 neighbouring pixels 7.6), and adds the patch to global memory once per
+// view, about half a pixel a sample.  The lanes are 32 slices of one column: they
+// fall on different rows, and where consecutive slices are at least a row apart
+// (checked per block and view) no two lanes hold the same pixel, so plain
+// additions serve, first to the samples' upper rows, then to the lower ones;
+// elsewhere shared-memory reductions (4.1 cycles each).  Samples outside the patch
+// (it holds kPatch pixels; a sample on the last column has no right neighbour)
+// go to global memory by themselves.  What bounds it is the shared memory: 20
+// wavefronts a sample, eight of them bank conflicts (32 lanes spread over more
+// than 32 rows).
+constexpr int kPatch = 1024, kAdjCols = 64, kAdjWarps = 4, kAdjBatch = 4;
+struct AdjWarp {
+    float patch[kPatch];
+    float rt[kAdjCols * 33];          // [column][slice], padded
+    float4 xy[kAdjCols];              // U, V, W at z = 0 and RN(1 / W) of the view
+};
 
 template <bool WZ, bool INSIDE>
 __device__ __forceinline__ void adjoint_views(const AdjParams& p, AdjWarp& m, const VoxelBox& box, int x0, int y0, int zb) {
@@ -464,7 +533,68 @@ __global__ void pad_rows_kernel(const float* __restrict__ src, int w, float* __r
 
 }  // namespace
 
-cudaError_t launch_bp_adjoint(const AdjParams& p, bool wz, cudaStream_t s) {
+// Whether a call's views go by patches: where that is the faster way, which is
+// where its plain additions run throughout.  The matrices (host copies, p.nv
+// views from h_ptm) tell for the whole volume that
+//   * it lies inside the detector (a block across the border runs without the
+//     plain additions: 256^3 with a fifth of its slices off the detector 3.7
+//     against 2.9 ms a 64-view chunk);
+//   * slices are more than a row apart (256^3 at 0.9 rows a slice at the far
+//     side: 5.4 against 3.7 ms, at 1.03 2.8 against 3.6);
+//   * a block fits its patch, or a sixteenth more than that by the extents
+//     below, which are those of the voxels nearest to the source: up to about
+//     1.4 pixels a voxel (1.45: 3.0 against 3.7 ms, 1.6: 4.1 against 3.8; 128^3
+//     0.58 against 0.60 and 0.92 against 0.62).
+// And the blocks, a warp each, have to be enough (6.5 per SM) and full (5/6): a
+// warp walks its views one after another, 0.43 ms for 64 however few the warps.
+// Where all hold, a chunk of 64 views takes 2.84 against 3.66 ms at 256^3, 1.31
+// against 1.64 at 192^3 and 0.53 against 0.59 at 128^3 (1.3 pixels a voxel); 96^3
+// (432 blocks) would take 0.45 against 0.26.
+bool adjoint_by_patches(const AdjParams& p, const float* h_ptm) {
+    const long long voxels = (long long)p.X * p.Y * p.Z, block = kAdjCols * 32;
+    const long long blocks = (long long)((p.X + 7) / 8) * ((p.Y + 7) / 8) * ((p.Z + 31) / 32);
+    if (2 * voxels < 13LL * p.sms * block || 6 * voxels < 5 * blocks * block) return false;
+    const float hx = 0.5f * (float)(p.X - 1) * p.pxy, hy = 0.5f * (float)(p.Y - 1) * p.pxy, hz = 0.5f * (float)(p.Z - 1) * p.pz;
+    const float ul = (float)(p.U - 1), vl = (float)(p.V - 1);
+    for (int n = 0; n < p.nv; ++n, h_ptm += 12) {
+        const float *r0 = h_ptm, *r1 = h_ptm + 4, *r2 = h_ptm + 8;
+        // least and largest of k r + l r2 over the volume
+        auto least = [&](const float* r, float k, float l) {
+            return k * r[3] + l * r2[3] - std::fabs(k * r[0] + l * r2[0]) * hx - std::fabs(k * r[1] + l * r2[1]) * hy -
+                   std::fabs(k * r[2] + l * r2[2]) * hz;
+        };
+        const float wmin = least(r2, 1.0f, 0.0f), wmax = -least(r2, -1.0f, 0.0f);
+        // (comparisons false for NaN)
+        if (!(wmin > 0.0f && least(r0, 1.0f, 0.49f) > 0.0f && least(r0, -1.0f, ul - 0.51f) > 0.0f &&
+              least(r1, 1.0f, 0.49f) > 0.0f && least(r1, -1.0f, vl - 0.51f) > 0.0f))
+            return false;
+        // du/dx = (P[0] - u P[8]) / W and its like, u over the detector
+        auto slope = [&](const float* r, int i, float lim) {
+            return std::max(std::fabs(r[i]), std::fabs(r[i] - lim * r2[i])) / wmin;
+        };
+        const float w = 7.0f * p.pxy * (slope(r0, 0, ul) + slope(r0, 1, ul)) + 31.0f * p.pz * slope(r0, 2, ul) + 2.1f;
+        const float h = 7.0f * p.pxy * (slope(r1, 0, vl) + slope(r1, 1, vl)) + 31.0f * p.pz * slope(r1, 2, vl) + 2.1f;
+        if (!(w * h <= 1.0625f * (float)kPatch)) return false;
+        if (!(p.pz * (std::fabs(r1[2]) - vl * std::fabs(r2[2])) > 1.01f * wmax)) return false;
+    }
+    return true;
+}
+
+cudaError_t launch_bp_adjoint_quads(const AdjParams& p, bool wz, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(p.quads, 0, sizeof(float4) * (size_t)p.nv * p.q_frame, s);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((p.X + 31) / 32, (p.Y + 7) / 8, (p.Z + kAdjZpt - 1) / kAdjZpt);
+    if (wz)
+        bp_adjoint_quads_kernel<true><<<grid, dim3(32, 8), 0, s>>>(p);
+    else
+        bp_adjoint_quads_kernel<false><<<grid, dim3(32, 8), 0, s>>>(p);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    unpack_adjoint_kernel<<<dim3((p.U + 255) / 256, std::min(p.V, 65535), std::min(p.nv, 65535)), 256, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bp_adjoint_patches(const AdjParams& p, bool wz, cudaStream_t s) {
     constexpr int smem = kAdjWarps * (int)sizeof(AdjWarp);
     // (per call: the attribute belongs to the current device)
     cudaError_t e = wz ? cudaFuncSetAttribute(bp_adjoint_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)

@@ -568,7 +568,7 @@ void jfdk_destroy(jfdk_ctx* c) {
     dev_free(c, c->d_plain);
     dev_free(c, c->d_q4); dev_free(c, c->d_qscale); dev_free(c, c->d_absmax);
     dev_free(c, c->d_sum); dev_free(c, c->d_cnt); dev_free(c, c->d_raw_stage); dev_free(c, c->d_hu_stage);
-    dev_free(c, c->d_Tt); dev_free(c, c->d_partial);
+    dev_free(c, c->d_Tt); dev_free(c, c->d_qadj); dev_free(c, c->d_partial);
     dev_free(c, c->d_dptm);
     dev_free(c, c->d_wvol);
     for (auto& e : c->ev)
@@ -1242,7 +1242,26 @@ jfdk_status jfdk_bp_adjoint(jfdk_ctx* c, const float* d_vol_bar, int v0, int nv,
     if (st || nv == 0) return st;
     AdjParams a = adj_params(c, d_vol_bar, v0, nv);
     a.qbar = d_q_bar;
-    JFDK_LAUNCH(c, launch_bp_adjoint(a, c->w_depends_on_z, c->stream), "backprojection adjoint");
+    // quad space where it is faster and its scratch is there or can be had (an
+    // allocation would break a capture under way); patches need none
+    bool quads = !adjoint_by_patches(a, &c->ptms[(size_t)v0 * 12]);
+    if (quads && c->qadj_views < nv) {
+        quads = false;
+        if (!capturing(c->stream)) {
+            dev_free(c, c->d_qadj);
+            c->qadj_views = 0;
+            st = dev_alloc(c, &c->d_qadj, (size_t)nv * frame_px(c), "the quad-space adjoint");
+            if (st && st != JFDK_ERR_OOM) return st;
+            if ((quads = !st)) c->qadj_views = nv;
+        }
+    }
+    if (quads) {
+        a.quads = c->d_qadj;
+        JFDK_LAUNCH(c, launch_bp_adjoint_quads(a, c->w_depends_on_z, c->stream), "backprojection adjoint");
+        ++c->launches;   // back to pixels
+        return JFDK_OK;
+    }
+    JFDK_LAUNCH(c, launch_bp_adjoint_patches(a, c->w_depends_on_z, c->stream), "backprojection adjoint");
     return JFDK_OK;
 }
 

@@ -260,6 +260,7 @@ struct AdjParams {
     const float* vol_bar;    // [Z][Y][X] dL / dvol
     const float* cnt;        // [Z][Y][X] the forward's weights: rt = vol_bar / cnt
     float* qbar;             // adjoint out: detector pixels [nv][V][U]
+    float4* quads;           // adjoint by quad space: scratch [nv][V][U]
     long long q_frame;       // V * U
     const float4* q4;        // gradient: the forward's tapered quads [nv][V][U]
     const float2* tw;        // [views][U] taper pairs (w[c], RN(w[c+1] - w[c]))
@@ -268,7 +269,12 @@ struct AdjParams {
     float* partial;          // gradient: [nv][ctas][6] scratch
     int sms;
 };
-cudaError_t launch_bp_adjoint(const AdjParams& p, bool w_depends_on_z, cudaStream_t s);
+// The adjoint backprojection in quad space (p.quads) or by patches in shared
+// memory (no scratch); the same sums either way, of any scan.  adjoint_by_patches:
+// which is the faster one (h_ptm: the matrices of the call's views).
+bool adjoint_by_patches(const AdjParams& p, const float* h_ptm);
+cudaError_t launch_bp_adjoint_quads(const AdjParams& p, bool w_depends_on_z, cudaStream_t s);
+cudaError_t launch_bp_adjoint_patches(const AdjParams& p, bool w_depends_on_z, cudaStream_t s);
 size_t geometry_gradient_ctas(const AdjParams& p);
 cudaError_t launch_geometry_gradient(const AdjParams& p, bool w_depends_on_z, double* grad, cudaStream_t s);
 cudaError_t launch_pad_rows(const float* src, size_t rows, int w, float* dst, int pitch, cudaStream_t s);
@@ -345,6 +351,7 @@ struct jfdk_ctx {
     float* d_hu_stage = nullptr; size_t hu_stage_bytes = 0;
     bool bp_has_views = false;
     // derivatives (allocated on demand)
+    float4* d_qadj = nullptr; int qadj_views = 0;    // quad-space adjoint
     float* d_partial = nullptr; size_t partial_n = 0;
     float* d_dptm = nullptr; int dptm_views = 0;
 
