@@ -269,6 +269,23 @@ int view_chunk(const jfdk_ctx* c) {
     return (int)std::min<long long>(n, c->nviews);
 }
 
+// The buffers of a chunk of views (the weighted rows, and with plain the filtered
+// frames), for the context's whole chunk however few views the call has: the
+// first call of any size makes room for all later ones, so that their pointers
+// stay what a captured graph recorded and a capture allocates nothing.  *chunk:
+// the views there is room for, 32 where the device has none for the larger default.
+jfdk_status ensure_chunk(jfdk_ctx* c, bool plain, int* chunk) {
+    auto make = [&](int n) {
+        *chunk = n;
+        jfdk_status st = ensure_A(c, (size_t)n * c->rows);
+        if (!st && plain) st = ensure_plain(c, n);
+        return !st && plain && mixed(c) ? ensure_absmax(c, n) : st;
+    };
+    const int n = view_chunk(c);
+    const jfdk_status st = make(n);
+    return st == JFDK_ERR_OOM && !c->opt_view_chunk && n > kViewChunk ? make(kViewChunk) : st;
+}
+
 // How the backprojection's matrices make a sample's place depend on z.
 void classify_geometry(jfdk_ctx* c) {
     c->w_depends_on_z = c->u_depends_on_z = false;
@@ -459,15 +476,9 @@ jfdk_status filter_stage_range(jfdk_ctx* c, const uint16_t* d_raw, int vbeg, int
                     "reconstruct: filter input width must be the frame width or twice it (compositing)");
     jfdk_status st = ensure_Q4(c, c->nviews);
     if (st) return st;
-    if (!chunk) chunk = view_chunk(c);
-    st = ensure_A(c, (size_t)chunk * c->rows);
-    if (!st) st = ensure_plain(c, chunk);
-    if (st == JFDK_ERR_OOM && !c->opt_view_chunk && chunk > kViewChunk) {   // no room for the larger default
-        chunk = kViewChunk;
-        st = ensure_A(c, (size_t)chunk * c->rows);
-        if (!st) st = ensure_plain(c, chunk);
-    }
-    if (st) return st;
+    int room = 0;
+    if ((st = ensure_chunk(c, true, &room))) return st;
+    chunk = chunk ? std::min(chunk, room) : room;
     const size_t frame = (size_t)c->scan.num_dets_u * c->scan.num_dets_v;
     for (int v0 = vbeg; v0 < vend; v0 += chunk) {
         const int nv = std::min(chunk, vend - v0);
@@ -1004,12 +1015,8 @@ jfdk_status jfdk_filter_raw(jfdk_ctx* c, const uint16_t* d_raw, int v0, int nv, 
     if (c->in_w != c->used_u && !compositing(c))
         return fail(c, JFDK_ERR_UNSUPPORTED,
                     "filter_raw: filter input width must be the frame width or twice it (compositing)");
-    int chunk = std::min(view_chunk(c), nv);
-    jfdk_status st = ensure_A(c, (size_t)chunk * c->rows);
-    if (st == JFDK_ERR_OOM && !c->opt_view_chunk && chunk > kViewChunk) {
-        chunk = kViewChunk;
-        st = ensure_A(c, (size_t)chunk * c->rows);
-    }
+    int chunk = 0;
+    jfdk_status st = ensure_chunk(c, false, &chunk);
     if (st) return st;
     const size_t frame = (size_t)c->scan.num_dets_u * c->scan.num_dets_v;
     for (int a = v0; a < v0 + nv; a += chunk) {

@@ -1,0 +1,61 @@
+"""The filter stage's buffers: the first call of a context makes room for every
+later one, so that a captured graph's pointers stay valid and a capture has
+nothing to allocate, whichever entry point came first."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(form="fp32", views=48, u=40, v=24, stream=None):
+    import torch
+
+    from jenhine_b200.fdk import FDKEngine, ReconConfig, ScanConfig
+    from jenhine_b200.phantom import ScanGeometry
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    P = ScanGeometry(views, 500.0, 800.0, u, v, 2.0, 2.0, seed=2).ptms()
+    e = FDKEngine(ScanConfig(views, 500.0, 800.0, u, v, 2.0), ReconConfig(16, 16, 12, 2.0, 2.0), P, precision=form,
+                  stream=stream)
+    raw = np.random.default_rng(3).integers(200, 60000, (views, v, u), dtype=np.uint16)
+    return e, raw, torch.from_numpy(raw).cuda()
+
+
+@pytest.mark.parametrize("form", ["fp32", "mixed"])
+def test_the_first_call_makes_room_for_all(form):
+    e, host, raw = _engine(form)
+    e.filter_raw(raw, 0, 1)
+    held = e.device_bytes
+    e.filter_raw(raw, 0, raw.shape[0])
+    assert e.device_bytes == held
+    e, host, raw = _engine(form)
+    want = e.reconstruct_host(host)
+    held = e.device_bytes
+    np.testing.assert_array_equal(e.reconstruct(raw).cpu().numpy(), want)
+    e.filter_raw(raw, 0, raw.shape[0])
+    assert e.device_bytes == held
+
+
+def test_a_captured_call_outlives_larger_ones():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        e, _, raw = _engine(stream=s.cuda_stream)
+        torch.cuda.synchronize()
+        want = e.filter_raw(raw, 0, raw.shape[0]).clone()   # another context's answer
+        torch.cuda.synchronize()
+        e, _, raw = _engine(stream=s.cuda_stream)
+        torch.cuda.synchronize()
+        e.filter_raw(raw, 0, 1)
+        out = torch.empty_like(want)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            e.filter_raw(raw, 0, raw.shape[0], out=out)
+        e.reconstruct(raw)
+        out.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
