@@ -250,9 +250,10 @@ enum {
                                  middle between two floats, rounded either
                                  way), lerps fused into FMAs                    */
     JFDK_OPT_VIEW_CHUNK = 2,  /* views preprocessed + filtered per launch in
-                                 jfdk_reconstruct (default: 32, or as many as
-                                 make the pixels of 32 frames of 768 x 768 when
-                                 frames are smaller and no
+                                 jfdk_reconstruct (default: 32, or of smaller
+                                 frames as many as make the bytes of 32 frames
+                                 of 768 x 768, 151 MB of buffers, dealt evenly
+                                 over the rotation, when no
                                  JFDK_OPT_DEVICE_MEMORY_LIMIT is set;
                                  jfdk_reconstruct_host: 32)                      */
     JFDK_OPT_STAGE_TIMING = 3,/* 1: jfdk_reconstruct records CUDA events on its

@@ -70,11 +70,11 @@ template <class T>
 void dev_free(jfdk_ctx* c, T*& p) {
     if (p) {
         auto it = c->alloc_bytes.find(p);
-        if (it != c->alloc_bytes.end()) {
+        if (it != c->alloc_bytes.end()) {   // (else a part of d_stage: freed with it)
             c->dev_bytes -= (long long)it->second;
             c->alloc_bytes.erase(it);
+            cudaFree(p);
         }
-        cudaFree(p);
     }
     p = nullptr;
 }
@@ -83,21 +83,6 @@ void dev_free(jfdk_ctx* c, T*& p) {
 int a_pitch(const jfdk_ctx* c) { return (int)round_up(c->in_w, 64); }
 long long frame_px(const jfdk_ctx* c) { return (long long)c->rows * c->out_w; }
 
-jfdk_status ensure_A(jfdk_ctx* c, size_t rows) {
-    if (c->a_rows >= rows) return JFDK_OK;
-    dev_free(c, c->d_A);
-    dev_free(c, c->d_e);
-    dev_free(c, c->d_arow);
-    c->a_rows = 0;
-    // room for a high and a low part of up to 4 bytes each
-    jfdk_status st = dev_alloc(c, reinterpret_cast<float**>(&c->d_A), rows * a_pitch(c) * 2, "the weighted rows");
-    if (st) return st;
-    if ((st = dev_alloc(c, &c->d_e, rows, "the edge means"))) return st;
-    if ((st = dev_alloc(c, &c->d_arow, rows, "the row scales"))) return st;
-    c->a_rows = rows;
-    return JFDK_OK;
-}
-
 bool mixed(const jfdk_ctx* c) { return c->precision == JFDK_PRECISION_MIXED; }
 
 int ramp_kind(const jfdk_ctx* c) {
@@ -105,18 +90,48 @@ int ramp_kind(const jfdk_ctx* c) {
     return mixed(c) ? JFDK_RAMP_BF16X3 : JFDK_RAMP_I8X14;
 }
 
-// The A operand in the layout the chosen ramp product reads: the high part
-// at d_A, the low part after a_rows rows of it.
+int operand_kind(const jfdk_ctx* c) {
+    const int k = ramp_kind(c);
+    return k == JFDK_RAMP_TF32X3 ? AOUT_TF32X2
+           : k == JFDK_RAMP_BF16X3 ? AOUT_BF16X2
+           : k == JFDK_RAMP_FP16X3 ? AOUT_FP16X2
+           : k == JFDK_RAMP_I8X14 ? AOUT_I8X4 : AOUT_F32;
+}
+
+// Bytes of a weighted row with all its parts: four a sample, eight as two TF32
+// parts.
+size_t a_row_bytes(const jfdk_ctx* c) { return (size_t)a_pitch(c) * (operand_kind(c) == AOUT_TF32X2 ? 8 : 4); }
+size_t a_rows(const jfdk_ctx* c) { return c->a_bytes / a_row_bytes(c); }   // that d_A has room for
+
+jfdk_status ensure_A_bytes(jfdk_ctx* c, size_t bytes) {
+    if (c->a_bytes >= bytes) return JFDK_OK;
+    dev_free(c, c->d_A);
+    c->a_bytes = 0;
+    jfdk_status st = dev_alloc(c, reinterpret_cast<char**>(&c->d_A), bytes, "the weighted rows");
+    if (!st) c->a_bytes = bytes;
+    return st;
+}
+
+jfdk_status ensure_A(jfdk_ctx* c, size_t rows) {
+    jfdk_status st = ensure_A_bytes(c, rows * a_row_bytes(c));
+    if (st || c->e_rows >= rows) return st;
+    dev_free(c, c->d_e);
+    dev_free(c, c->d_arow);
+    c->e_rows = 0;
+    if ((st = dev_alloc(c, &c->d_e, rows, "the edge means"))) return st;
+    if ((st = dev_alloc(c, &c->d_arow, rows, "the row scales"))) return st;
+    c->e_rows = rows;
+    return JFDK_OK;
+}
+
+// The A operand in the layout the chosen ramp product reads: the parts one
+// behind the other, as many rows apart as d_A has room for.
 AOperand a_operand(const jfdk_ctx* c) {
     AOperand a{};
-    const int k = ramp_kind(c);
-    a.kind = k == JFDK_RAMP_TF32X3 ? AOUT_TF32X2
-             : k == JFDK_RAMP_BF16X3 ? AOUT_BF16X2
-             : k == JFDK_RAMP_FP16X3 ? AOUT_FP16X2
-             : k == JFDK_RAMP_I8X14 ? AOUT_I8X4 : AOUT_F32;
+    a.kind = operand_kind(c);
     const size_t elem = a.kind == AOUT_I8X4 ? 1 : (a.kind == AOUT_BF16X2 || a.kind == AOUT_FP16X2) ? 2 : 4;
     a.hi = c->d_A;
-    a.lo = static_cast<char*>(c->d_A) + c->a_rows * a_pitch(c) * elem;
+    a.lo = static_cast<char*>(c->d_A) + a_rows(c) * a_pitch(c) * elem;
     a.row_scale = c->d_arow;
     a.pitch = a_pitch(c);
     return a;
@@ -251,22 +266,45 @@ BPParams bp_params(const jfdk_ctx* c) {
     return b;
 }
 
-// Views preprocessed and filtered per launch: the option, else 32, or as many
-// as make the pixels of 32 frames of 768 x 768 when frames are smaller: the
-// weighted rows and filtered frames of a chunk (150 MB there) pass from kernel
-// to kernel through L2, while 32 small frames leave each launch one or two
-// rounds of tiles (360 frames of 256 x 256: 477 us of filter stage in 12 chunks
-// of 32, 337 in two of 288 and 72; a mixed reconstruction 1070 -> 839 us).  A
-// context with a bound on its device memory keeps to 32.
+// Views preprocessed and filtered per launch: the option, else 32, or of smaller
+// frames as many as make the bytes of 32 frames of 768 x 768 (4 of weighted rows,
+// their padding counted, and 4 of filtered frames a pixel: 151 MB), dealt evenly
+// over the rotation.  A chunk's buffers pass from kernel to kernel through L2,
+// while 32 small frames leave each launch one or two rounds of tiles: a mixed
+// 128^3 volume from 360 frames of 256 x 256 takes 989 us in chunks of 32, 902 of
+// 64, 854 of 120 and 824 of 180 (what the rule gives: 94 MB; 809 in one of 360).
+// A context with a bound on its device memory keeps to 32.
 constexpr int kViewChunk = 32;
 int view_chunk(const jfdk_ctx* c) {
-    long long n = c->opt_view_chunk;
-    if (!n) {
-        n = kViewChunk;
-        if (c->mem_limit <= 0)
-            n = std::min(4096LL, std::max(n, 32LL * 768 * 768 / ((long long)c->rows * std::max(c->in_w, c->out_w))));
+    if (c->opt_view_chunk) return std::min(c->opt_view_chunk, c->nviews);
+    long long n = kViewChunk;
+    if (c->mem_limit <= 0) {
+        const long long frame = (long long)c->rows * (long long)(a_row_bytes(c) + c->out_w * sizeof(float));
+        n = std::min(4096LL, std::max(n, 32LL * 768 * 768 * 8 / frame));
+    }
+    if (n > kViewChunk) {
+        const long long chunks = (c->nviews + n - 1) / n;
+        n = std::max<long long>(kViewChunk, (c->nviews + chunks - 1) / chunks);
     }
     return (int)std::min<long long>(n, c->nviews);
+}
+
+// The store, the weighted rows and the filtered frames of a context that has
+// none of them yet, in one allocation (d_stage, of which they are parts): the first
+// reconstruction then waits for one cudaMalloc in place of three, 0.3 ms each (256 x
+// 256 x 360 frames 2.9 -> 2.2 ms).  No room in one piece: nothing, and each is allocated by itself.
+void stage_once(jfdk_ctx* c) {
+    if (c->d_stage || c->d_q4 || c->d_A || c->d_plain) return;
+    const int n = view_chunk(c);
+    const size_t store = round_up((size_t)c->nviews * frame_px(c) * record_size(c), 256);
+    const size_t a = round_up((size_t)n * c->rows * a_row_bytes(c), 256);
+    if (dev_alloc(c, &c->d_stage, store + a + (size_t)n * frame_px(c) * sizeof(float), "the filter stage")) return;
+    c->d_q4 = reinterpret_cast<float4*>(c->d_stage);
+    c->q4_views = c->nviews;
+    c->d_A = c->d_stage + store;
+    c->a_bytes = a;
+    c->d_plain = reinterpret_cast<float*>(c->d_stage + store + a);
+    c->plain_views = n;
 }
 
 // The buffers of a chunk of views (the weighted rows, and with plain the filtered
@@ -474,6 +512,7 @@ jfdk_status filter_stage_range(jfdk_ctx* c, const uint16_t* d_raw, int vbeg, int
     if (c->in_w != c->used_u && !compositing(c))
         return fail(c, JFDK_ERR_UNSUPPORTED,
                     "reconstruct: filter input width must be the frame width or twice it (compositing)");
+    stage_once(c);
     jfdk_status st = ensure_Q4(c, c->nviews);
     if (st) return st;
     int room = 0;
@@ -577,7 +616,7 @@ void jfdk_destroy(jfdk_ctx* c) {
     dev_free(c, c->d_Ti8); dev_free(c, c->d_i8mask);
     dev_free(c, c->d_status); dev_free(c, c->d_c); dev_free(c, c->d_c64); dev_free(c, c->d_A); dev_free(c, c->d_e); dev_free(c, c->d_arow);
     dev_free(c, c->d_plain);
-    dev_free(c, c->d_q4); dev_free(c, c->d_qscale); dev_free(c, c->d_absmax);
+    dev_free(c, c->d_q4); dev_free(c, c->d_stage); dev_free(c, c->d_qscale); dev_free(c, c->d_absmax);
     dev_free(c, c->d_sum); dev_free(c, c->d_cnt); dev_free(c, c->d_raw_stage); dev_free(c, c->d_hu_stage);
     dev_free(c, c->d_Tt); dev_free(c, c->d_qadj); dev_free(c, c->d_partial);
     dev_free(c, c->d_dptm);
@@ -1278,7 +1317,7 @@ jfdk_status jfdk_filter_adjoint(jfdk_ctx* c, const float* d_q_bar, int v0, int n
     const int kp = (int)round_up(c->out_w, 64);
     const size_t m = (size_t)nv * c->rows;
     // the padded rows of q_bar go where the forward keeps its A operand
-    jfdk_status st = ensure_A(c, (m * kp + 2 * a_pitch(c) - 1) / (2 * a_pitch(c)));
+    jfdk_status st = ensure_A_bytes(c, m * kp * sizeof(float));
     if (st) return st;
     float* ypad = static_cast<float*>(c->d_A);
     JFDK_LAUNCH(c, launch_pad_rows(d_q_bar, m, c->out_w, ypad, kp, c->stream), "filter adjoint (pad)");

@@ -336,9 +336,10 @@ struct jfdk_ctx {
     int* d_status = nullptr;     // nonzero: a kernel's bounded wait gave up
 
     // device working storage (allocated on demand)
-    void* d_A = nullptr;  size_t a_rows = 0;    // weighted rows: high then low part, pitch a_pitch
+    char* d_stage = nullptr;                     // one allocation for d_q4, d_A and d_plain (stage_once), or none
+    void* d_A = nullptr;  size_t a_bytes = 0;    // weighted rows: high then low part, pitch a_pitch
     float* d_arow = nullptr;                     // FP16X3: per-row factors
-    float* d_e = nullptr;
+    float* d_e = nullptr; size_t e_rows = 0;     // rows d_e and d_arow have room for
     float* d_plain = nullptr; int plain_views = 0;  // filtered frames of one chunk
     float4* d_q4 = nullptr; int q4_views = 0;       // quad store (mixed: 8-byte records)
     float* d_qscale = nullptr;                      // mixed: [views] scales

@@ -59,3 +59,41 @@ def test_a_captured_call_outlives_larger_ones():
         g.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("views,u,v", [(700, 256, 256), (400, 33, 256), (90, 64, 64), (40, 768, 768)])
+def test_a_chunk_is_bounded_and_dealt_evenly(views, u, v):
+    """At most the bytes of 32 frames of 768 x 768 (8 a pixel, rows of weighted samples
+    padded to 64), and chunks that differ by less than their number."""
+    import torch
+
+    from jenhine_b200 import _lib
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    e, _, raw = _engine(views=views, u=u, v=v)
+    chunk = e.get_option(_lib.OPT_VIEW_CHUNK)
+    last = (views - 1) % chunk + 1
+    assert chunk == min(views, 32) or chunk - last < -(-views // chunk)
+    before = e.device_bytes
+    e.reconstruct(raw)
+    held = e.device_bytes - before - 16 * views * u * v - 4 * 16 * 16 * 12
+    row = 4 * (-(-u // 64) * 64 + u)
+    assert held <= chunk * v * (row + 8) + 4096
+    assert chunk == min(views, 32) or chunk * v * row <= 32 * 768 * 768 * 8
+
+
+def test_another_product_in_the_same_buffers():
+    """The parts of the weighted rows take 4 or 8 bytes a sample: a context that changes
+    its ramp product gives what one with that product from the start gives."""
+    import torch
+
+    from jenhine_b200 import _lib
+    e, _, raw = _engine(u=70)
+    want = {}
+    for product in (_lib.RAMP_I8X14, _lib.RAMP_TF32X3, _lib.RAMP_FP16X3, _lib.RAMP_FP32_SIMT, _lib.RAMP_BF16X3):
+        f, _, _ = _engine(u=70)
+        f.set_option(_lib.OPT_RAMP_PRODUCT, product)
+        want[product] = f.reconstruct(raw)
+    for product in (*want, *reversed(want)):
+        e.set_option(_lib.OPT_RAMP_PRODUCT, product)
+        assert torch.equal(e.reconstruct(raw).nan_to_num(1e30), want[product].nan_to_num(1e30)), product
