@@ -255,7 +255,7 @@ enum {
                                  of 768 x 768, 151 MB of buffers, dealt evenly
                                  over the rotation, when no
                                  JFDK_OPT_DEVICE_MEMORY_LIMIT is set;
-                                 jfdk_reconstruct_host: 32)                      */
+                                 jfdk_reconstruct_host: 32); 0 sets the default  */
     JFDK_OPT_STAGE_TIMING = 3,/* 1: jfdk_reconstruct records CUDA events on its
                                  stream around each stage                        */
     JFDK_OPT_BP_ZPT = 4,      /* slices each backprojection thread keeps in
@@ -354,11 +354,11 @@ jfdk_status jfdk_geometry_gradient(jfdk_ctx* ctx, const float* d_q, int v0, int 
 
 /* Pick the backprojection's voxel tile (JFDK_OPT_BP_ZPT: 4 or 8 slices per
  * thread, and 16 in the mixed form; JFDK_OPT_BP_TILE: 4, 8 or 32 threads wide
- * in x, 128 per CTA, 16-slice tiles 4 wide) and
- * the filter stage's views per chunk (JFDK_OPT_VIEW_CHUNK: 16, 32 or 64, 64 leaving the
- * default where that is more) for
- * this context's shape by timing the candidates on the device (a 32-slice
- * slab, the first 128 views of zero frames).  Results are cached per shape in the process and, when
+ * in x, 128 per CTA, 16-slice tiles 4 wide) and the filter stage's views per
+ * chunk (JFDK_OPT_VIEW_CHUNK: the default, or 16, 32 or 64 where that is 2 %
+ * faster; unchanged with compositing) for this context's shape by timing the
+ * candidates on the device (a 32-slice slab, zero frames of 128 views or two
+ * chunks).  Results are cached per shape in the process and, when
  * $JFDK_AUTOTUNE_CACHE names a file, appended to it and read back by later
  * processes.  Synchronises the context's stream. */
 enum { JFDK_AUTOTUNE_FORCE = 1 };  /* re-time even when the shape is cached */

@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <iterator>
 #include <map>
 #include <mutex>
 #include <cstdio>
@@ -840,7 +841,7 @@ jfdk_status jfdk_set_option(jfdk_ctx* c, int key, long long value) {
     switch (key) {
         case JFDK_OPT_BP_EXACT: c->opt_bp_exact = value ? 1 : 0; return JFDK_OK;
         case JFDK_OPT_VIEW_CHUNK:
-            if (value < 1 || value > 4096) return fail(c, JFDK_ERR_INVALID, "view chunk out of range");
+            if (value < 0 || value > 4096) return fail(c, JFDK_ERR_INVALID, "view chunk out of range");
             c->opt_view_chunk = (int)value;
             return JFDK_OK;
         case JFDK_OPT_BP_ZPT:
@@ -1369,7 +1370,7 @@ namespace {
 
 std::mutex g_tune_mutex;
 struct TuneChoice {
-    int zpt, chunk, tile;   // slices per thread, views per chunk, tile width in x
+    int zpt, chunk, tile;   // slices per thread, views per chunk (0: the default), tile width in x
 };
 std::map<std::string, TuneChoice> g_tune_cache;   // shape -> choice
 bool g_tune_file_read = false;
@@ -1382,7 +1383,11 @@ std::string tune_key(const jfdk_ctx* c) {
 }
 
 // Optional persistent cache: $JFDK_AUTOTUNE_CACHE, lines "key zpt chunk tile"
-// (lines without the tile width, from earlier builds, read as width 4).
+// (lines without the tile width, from earlier builds, read as width 4).  The
+// default views per chunk stand there as the candidate that comes to the same
+// number, or as 0.
+constexpr int kChunks[] = {16, 32, 64};
+bool known_chunk(int ch) { return std::find(std::begin(kChunks), std::end(kChunks), ch) != std::end(kChunks); }
 void tune_file_load() {
     if (g_tune_file_read) return;
     g_tune_file_read = true;
@@ -1394,7 +1399,7 @@ void tune_file_load() {
     while (std::fgets(line, sizeof line, f)) {
         int z = 0, ch = 0, tx = kBPTileX;
         if (std::sscanf(line, "%255s %d %d %d", key, &z, &ch, &tx) < 3) continue;
-        if ((z == 4 || z == 8 || z == 16) && (ch == 16 || ch == 32 || ch == 64) && (tx == 4 || tx == 8 || tx == 32))
+        if ((z == 4 || z == 8 || z == 16) && (ch == 0 || known_chunk(ch)) && (tx == 4 || tx == 8 || tx == 32))
             g_tune_cache[key] = {z, ch, tx};
     }
     std::fclose(f);
@@ -1409,11 +1414,11 @@ void tune_file_append(const std::string& key, const TuneChoice& t) {
     std::fclose(f);
 }
 
-// The tuned views per chunk; the largest candidate stands for "as many as the
-// frame size calls for" where that is more.
+// Whether views per chunk are tuned: not with compositing, which reads conjugate
+// frames of the whole rotation.  Untuned, the option stays as it is.
+bool tunes_chunk(const jfdk_ctx* c) { return c->in_w == c->used_u; }
 void take_chunk(jfdk_ctx* c, int chunk) {
-    c->opt_view_chunk = 0;
-    if (chunk != 64 || view_chunk(c) <= 64) c->opt_view_chunk = chunk;
+    if (tunes_chunk(c)) c->opt_view_chunk = chunk;
 }
 
 // The smaller of two timed runs after one warm-up run.
@@ -1490,29 +1495,41 @@ extern "C" jfdk_status jfdk_autotune(jfdk_ctx* c, int flags) {
     if (st) return st;
     c->opt_bp_zpt = best_z;
     c->opt_bp_tile = best_x;
-    // views per chunk: the filter stage over the first views of zero frames
-    int best_c = c->opt_view_chunk ? c->opt_view_chunk : kViewChunk;
-    if (c->in_w == c->used_u) {   // (compositing reads conjugate frames of the whole rotation)
-        const int nsub = std::min(c->nviews, 128);
+    // views per chunk: the filter stage over the first views of zero frames, the
+    // default first; another number only where it is 2 % faster than that
+    int best_c = 0, line_c = 0;
+    if (tunes_chunk(c)) {
+        const int before = c->opt_view_chunk;
+        c->opt_view_chunk = 0;
+        const int usual = view_chunk(c);
+        const int nsub = std::min(c->nviews, std::max(128, 2 * usual));
         uint16_t* raw = nullptr;
         const size_t frame = (size_t)c->scan.num_dets_u * c->scan.num_dets_v;
-        if ((st = dev_alloc(c, &raw, frame * nsub, "the autotuner's frames"))) return st;
-        JFDK_CUDA(c, cudaMemsetAsync(raw, 0, frame * nsub * sizeof(uint16_t), c->stream), "autotune");
+        st = dev_alloc(c, &raw, frame * nsub, "the autotuner's frames");
+        if (!st && cudaMemsetAsync(raw, 0, frame * nsub * sizeof(uint16_t), c->stream) != cudaSuccess)
+            st = cuda_fail(c, cudaGetLastError(), "autotune");
         best_t = 1e30f;
-        for (int ch : {16, 32, 64}) {
+        for (int ch : {0, kChunks[0], kChunks[1], kChunks[2]}) {
+            if (st) break;
+            if (ch && std::min(ch, c->nviews) == usual) {   // the default by another name
+                line_c = ch;
+                continue;
+            }
             c->opt_view_chunk = ch;
             float t = 0.0f;
             st = time_ms(c, [&] { return jfdk::reconstruct_filter_stage(c, raw, nsub); }, &t);
             if (st) break;
-            if (t < best_t) { best_t = t; best_c = ch; }
+            if (t < best_t) { best_t = ch ? t : 0.98f * t; best_c = ch; }
         }
         cudaStreamSynchronize(c->stream);
         dev_free(c, raw);
+        c->opt_view_chunk = before;
         if (st) return st;
+        if (best_c) line_c = best_c;
     }
     take_chunk(c, best_c);
     std::lock_guard<std::mutex> lk(g_tune_mutex);
     g_tune_cache[key] = {best_z, best_c, best_x};
-    tune_file_append(key, g_tune_cache[key]);
+    tune_file_append(key, {best_z, line_c, best_x});
     return JFDK_OK;
 }
