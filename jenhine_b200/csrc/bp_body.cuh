@@ -59,12 +59,21 @@ constexpr int kBPThreads = kBPTileX * kBPTileY;
 //
 // FP32, 8 slices: 80 registers and 24 warps per SM with two views in flight,
 // 111.0 ms a c2 volume (96 registers and 20 warps 112.3; one view at a time
-// 114.2).  Mixed, 16 slices (the default on large volumes when W does not
-// depend on z): 128 registers and 16 warps, 81.2 ms (96 registers and 20 warps
-// spill: 82.5; 80 and 24, one view at a time: 83.7); 8 slices: 72 registers and
-// 28 warps, 1070 us a 128^3 volume (64 and 32: 1103; 80 and 24: 1196).
+// 114.2).  Mixed: bp_mixed_kernel's launches choose (bp_mixed.cu); these are the
+// weights' and the batch kernel's.
 constexpr int bp_min_blocks(int zpt) { return zpt == 8 ? 7 : zpt == 16 ? 4 : 1; }
 constexpr int bp_fp32_min_blocks(int zpt) { return zpt == 8 ? 6 : 1; }
+
+// Least views of a launch that asks where its tiles lie (tile_inside): a CTA waits
+// for the matrices before its first sample, which few views do not earn back
+// (640 x 640 x 480 voxels from one view 1112 us with it and 1069 without, two 1301
+// and 1250, four 1684 and 1696; mixed 8-slice tiles 256 x 256 x 160 from one 69.7
+// and 67.7, two 76.5 and 81).  On an ideal orbit, and with 16 mixed slices a
+// thread, the loops with the range test are the slower ones from the first view on;
+// with W(z) the choice costs the loops of more views what it saves (one view 65.6
+// and 63.6 us, 24 386 and 391).
+constexpr int box_views_fp32(int geo) { return geo == kGeoWConst ? 4 : 0; }
+constexpr int box_views_mixed(int zpt) { return zpt == 16 ? 0 : 2; }
 
 // Where a CTA's tile lies: the launch grid's block index for the per-scan
 // kernels, the current work item of the batch kernel.  The tile bodies ask
@@ -311,11 +320,12 @@ template <int ZPT, bool FINALIZE, bool EXACT, int G, class Tile, bool WV = false
           bool SPLIT = true, bool WIDE = false>
 __device__ __forceinline__ void bp_block(const BPParams& p, const Tile& tile, float* wout = nullptr) {
     unsigned* none = nullptr;
-    bool inside = false;
+    bool asked = false, inside = false;
     if constexpr (SPLIT) {
         __shared__ unsigned none_bits[kNoneViews / 32];
         none = none_bits;
-        inside = tile_inside<ZPT>(p, tile, none);
+        asked = box_views_fp32(G) == 0 || p.nv >= box_views_fp32(G);
+        if (asked) inside = tile_inside<ZPT>(p, tile, none);
     }
     const int x = tile.bx() * Tile::kX + threadIdx.x;
     const int y = tile.by() * Tile::kY + threadIdx.y;
@@ -336,7 +346,7 @@ __device__ __forceinline__ void bp_block(const BPParams& p, const Tile& tile, fl
     }
     if (SPLIT && inside)
         bp_views<ZPT, EXACT, G, WV, WEIGHTS, true, WIDE>(p, none, ax, ay, az, acc);
-    else if (SPLIT && any_none(none, p.nv))
+    else if (SPLIT && asked && any_none(none, p.nv))
         bp_views<ZPT, EXACT, G, WV, WEIGHTS, false, WIDE, SPLIT>(p, none, ax, ay, az, acc);
     else
         bp_views<ZPT, EXACT, G, WV, WEIGHTS, false, WIDE>(p, none, ax, ay, az, acc);
@@ -506,11 +516,12 @@ template <int ZPT, bool FINALIZE, int G, class Tile, bool WV = false, bool WEIGH
           bool WIDE = false>
 __device__ __forceinline__ void bp_mixed_block(const BPParams& p, const Tile& tile, float* wout = nullptr) {
     unsigned* none = nullptr;
-    bool inside = false;
+    bool asked = false, inside = false;
     if constexpr (SPLIT) {
         __shared__ unsigned none_bits[kNoneViews / 32];
         none = none_bits;
-        inside = tile_inside<ZPT>(p, tile, none);
+        asked = box_views_mixed(ZPT) == 0 || p.nv >= box_views_mixed(ZPT);
+        if (asked) inside = tile_inside<ZPT>(p, tile, none);
     }
     const int x = tile.bx() * Tile::kX + threadIdx.x;
     const int y = tile.by() * Tile::kY + threadIdx.y;
@@ -532,7 +543,7 @@ __device__ __forceinline__ void bp_mixed_block(const BPParams& p, const Tile& ti
     }
     if (SPLIT && inside)
         bp_mixed_views<ZPT, G, WV, WEIGHTS, true, WIDE>(p, none, ax, ay, az0, acc);
-    else if (SPLIT && any_none(none, p.nv))
+    else if (SPLIT && asked && any_none(none, p.nv))
         bp_mixed_views<ZPT, G, WV, WEIGHTS, false, WIDE, SPLIT>(p, none, ax, ay, az0, acc);
     else
         bp_mixed_views<ZPT, G, WV, WEIGHTS, false, WIDE>(p, none, ax, ay, az0, acc);

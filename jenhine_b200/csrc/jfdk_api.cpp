@@ -447,7 +447,7 @@ jfdk_status run_bp_on(jfdk_ctx* c, BPParams b, bool finalize, cudaStream_t s) {
     if (mixed(c)) {
         b.qh = reinterpret_cast<const uint2*>(c->d_q4);
         b.qscale = c->d_qscale;
-        JFDK_LAUNCH(c, launch_bp_mixed(b, finalize, geometry(c), bp_zpt(c), bp_tile(c), s), "backprojection");
+        JFDK_LAUNCH(c, launch_bp_mixed(b, finalize, geometry(c), bp_zpt(c), bp_tile(c), c->sms, s), "backprojection");
         return JFDK_OK;
     }
     JFDK_LAUNCH(c, launch_bp(b, finalize, c->opt_bp_exact != 0, geometry(c), launch_zpt(c, b.z_end - b.z_begin), bp_tile(c), s),

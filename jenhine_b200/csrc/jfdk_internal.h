@@ -133,7 +133,7 @@ cudaError_t bp_batch_ctas(bool mixed_form, bool wz, bool wv, bool deep, int* cta
 // The context's backprojection store for every view (allocated if missing).
 jfdk_status ensure_store(jfdk_ctx* c);
 // Mixed-precision form: FP16 footprints with a per-view scale (qh, qscale).
-cudaError_t launch_bp_mixed(const BPParams& p, bool finalize, Geo geo, int zpt, int tile_x,
+cudaError_t launch_bp_mixed(const BPParams& p, bool finalize, Geo geo, int zpt, int tile_x, int sms,
                             cudaStream_t s);
 // absmax[f] = bit pattern of max |plain[f][...]| over each of nv frames.
 cudaError_t launch_frame_absmax(const float* plain, long long frame, int nv, unsigned* absmax, cudaStream_t s);
