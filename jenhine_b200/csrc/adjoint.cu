@@ -347,6 +347,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 4) bp_adjoint_kernel(AdjParams
 // 3.2; 3.26 with the reduction every 8 samples, 32 x 1 warps and 64 registers).
 // J is 1 where 4 would leave less than a full wave of CTAs.
 constexpr int kGradThreads = 128, kGradRows = kGradThreads / 8;   // 8 columns x kGradRows of warps of 4 x 8
+constexpr int kGradRed = 2 * (kGradThreads / 32) * 16;           // floats the CTA's reduction takes, double buffered
 
 template <int J, bool WZ, bool INSIDE>
 __device__ __forceinline__ void gradient_views(const AdjParams& p, const float2* vox, float* red, int x0, int y, int zb) {
@@ -451,7 +452,7 @@ template <int J, bool WZ>
 __global__ void __launch_bounds__(kGradThreads, 4) geometry_gradient_kernel(AdjParams p) {
     constexpr int ZPT = kAdjZpt;
     extern __shared__ float2 vox[];            // [J][ZPT][kGradThreads] (rt, vol)
-    __shared__ float red[2 * (kGradThreads / 32) * 16];
+    __shared__ float red[kGradRed];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int xb = blockIdx.x * 8 * J, yb = blockIdx.y * kGradRows, zb = blockIdx.z * ZPT;
     const int x0 = xb + (warp & 1) * 4 + (lane & 3), y = yb + (warp >> 1) * 8 + (lane >> 2);
@@ -626,11 +627,7 @@ bool gradient_deep(const AdjParams& p) { return blocks_of(gradient_grid<4>(p)) >
 template <int J, bool WZ>
 cudaError_t go_gradient(const AdjParams& p, cudaStream_t s) {
     constexpr int smem = J * kAdjZpt * kGradThreads * (int)sizeof(float2);
-    if constexpr (smem > 32 * 1024) {   // per call: the attribute belongs to the current device
-        const cudaError_t e = cudaFuncSetAttribute(geometry_gradient_kernel<J, WZ>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-    }
+    static_assert(smem + kGradRed * (int)sizeof(float) <= 48 * 1024, "shared memory without an attribute");
     geometry_gradient_kernel<J, WZ><<<gradient_grid<J>(p), kGradThreads, smem, s>>>(p);
     return cudaGetLastError();
 }

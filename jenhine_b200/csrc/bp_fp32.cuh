@@ -29,12 +29,10 @@ cudaError_t go(const BPParams& p, cudaStream_t s) {
 // (4 and 8 slices); 16-slice tiles are 4 wide.
 template <int ZPT, bool F, bool E, int G>
 cudaError_t go_tx(const BPParams& p, int tx, cudaStream_t s) {
-#ifndef DEV
     if constexpr (ZPT != 16) {
         if (tx == 8) return go<ZPT, F, E, G, 8>(p, s);
         if (tx == 32) return go<ZPT, F, E, G, 32>(p, s);
     }
-#endif
     return go<ZPT, F, E, G, 4>(p, s);
 }
 
