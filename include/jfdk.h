@@ -246,7 +246,7 @@ enum {
     JFDK_OPT_BP_EXACT = 1,    /* FP32 form.  1: backprojection rounds every
                                  step like BPCore (bit-identical sums);
                                  0 (default): the same sample coordinates (but
-                                 for quotients that lie within 2^-47 of the
+                                 for quotients that lie within 3 2^-48 of the
                                  middle between two floats, rounded either
                                  way), lerps fused into FMAs                    */
     JFDK_OPT_VIEW_CHUNK = 2,  /* views preprocessed + filtered per launch in

@@ -13,8 +13,10 @@
 //     with u = U/W, du/dtheta_j = (dU_j - u dW_j) / W for (dU_j, dV_j, dW_j)
 //     = (dP/dtheta_j) X; per-CTA partial sums in FP32, the reduction over
 //     CTAs in FP64.
-// Every kernel uses the forward's sample points and in-range decisions
-// (bp_common.cuh), so the adjoint is the transpose of the forward as computed.
+// Every kernel uses the default form's sample points and in-range decisions
+// (bp_common.cuh), so the adjoint is the transpose of the forward as computed (of
+// one with JFDK_OPT_BP_EXACT but for the quotients that bp_quotient2 rounds the
+// other way).
 #include <cuda_runtime.h>
 
 #include <algorithm>

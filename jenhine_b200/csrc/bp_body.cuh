@@ -9,7 +9,8 @@
 //     image of the taper is backprojected alongside it (the weight);
 //   * for voxel (x, y, z): U = (x*P0 + (y*P1 + P3)) + z*P2, likewise V, W,
 //     every product and sum rounded separately; u = U / W + 0.5,
-//     v = V / W + 0.5 with the quotient correctly rounded;
+//     v = V / W + 0.5 with the quotient correctly rounded (in the default form but
+//     for a few in 10^9, bp_quotient2);
 //   * bilinear sample with pixel centres at integers, taken only when
 //     0 <= u <= cols-1 and 0 <= v <= rows-1 (ippiRemap leaves the destination
 //     untouched otherwise, so the view then adds nothing to sum or weight);

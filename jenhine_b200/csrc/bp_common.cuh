@@ -104,7 +104,8 @@ __device__ __forceinline__ float rcp_rn_nr(float w) {
 }
 
 // 1/W as a float r = RN(1/W) and the float nearest to what r lacks, rl =
-// RN(RN(1 - W r) r): the residual 1 - W r is exact, so r + rl is 1/W to 2^-47.
+// RN(e r) with e = 1 - W r, which is exact and at most 2^-24: r + rl is within
+// 2^-47 of 1/W, e^2 left out and rl rounded being 2^-48 each.
 struct Recip { float r, rl; };
 
 __device__ __forceinline__ Recip bp_recip(float W) {
@@ -114,11 +115,14 @@ __device__ __forceinline__ Recip bp_recip(float W) {
 
 // U / W of both lanes.  EXACT: correctly rounded, from r and Markstein's
 // correction q = RN(q0 + RN(U - W q0) r), q0 = RN(U r).  Otherwise
-// RN(U r + RN(U rl)), one operation less (5 % of the FP32 loop): the sum is within 2^-47 of U / W
-// before its one rounding, so it is the correctly rounded quotient but where
-// U / W lies that close to the middle between two floats (none of 1.6e8 random
-// quotients), and then the other of the two, off by half a unit in the last
-// place like the one it stands for.
+// RN(U r + RN(U rl)), one operation less (5 % of the FP32 loop): the sum is
+// within 3 2^-48 of U / W before its one rounding (a third 2^-48 from RN(U rl)), so
+// it is the correctly rounded quotient but where U / W lies that close to the
+// middle between two floats, and then the other of the two, off by half a unit in
+// the last place like the one it stands for: 5 of 2.1e9 random quotients
+// (tests/cuda/quotient_check.cu).  This holds while rl and U rl stay normal: |W|
+// from 2^-78 to 2^78, |U / W| above 2^-78, far below what the 0.5 that a place adds
+// leaves of it.
 template <bool EXACT>
 __device__ __forceinline__ float2 bp_quotient2(float2 U, float W, const Recip& rc) {
     const float2 rr = f2(rc.r, rc.r);
