@@ -9,12 +9,13 @@ __global__ void __launch_bounds__(kBPThreads, bp_fp32_min_blocks(ZPT)) bp_weight
     bp_block<ZPT, true, EXACT, WZ ? kGeoWZ : kGeoWConst, GridTile<TX>, false, true>(p, GridTile<TX>{}, out);
 }
 
-// (once per geometry; with 16 slices at 128 registers, which the weights'
-// taper lerps fill without spilling)
+// (once per geometry; with 16 slices at 128 registers.  Tiles inside the detector
+// run without the range test as in the backprojection: 640 x 640 x 480 voxels from
+// 600 views 53.0 ms, all tiles by the range test 82.6)
 template <int ZPT, bool WZ, int TX>
 __global__ void __launch_bounds__(kBPThreads, ZPT == 16 ? 4 : bp_min_blocks(ZPT))
     bp_mixed_weights_kernel(BPParams p, float* out) {
-    bp_mixed_block<ZPT, true, WZ ? kGeoWZ : kGeoWConst, GridTile<TX>, false, true, false>(p, GridTile<TX>{}, out);
+    bp_mixed_block<ZPT, true, WZ ? kGeoWZ : kGeoWConst, GridTile<TX>, false, true>(p, GridTile<TX>{}, out);
 }
 
 template <int ZPT, bool E, bool WZ>
