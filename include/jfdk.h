@@ -261,11 +261,12 @@ enum {
     JFDK_OPT_BP_ZPT = 4,      /* slices each backprojection thread keeps in
                                  registers: 4, 8 or 16; 0 (default): 16 in the
                                  mixed form when W does not depend on z and the
-                                 volume holds at least 8 waves of 16-slice
-                                 tiles (c2 does, c1 does not), else 8.
-                                 The FP32 form's volume does not depend on it;
-                                 the mixed form's coordinates step from each
-                                 tile's first slice, so its volume does      */
+                                 volume holds at least 40 16-slice tiles per SM
+                                 (c2 does, c1 does not), else 8.
+                                 The FP32 form's volume does not depend on it,
+                                 and small launches of its default run 4; the
+                                 mixed form's coordinates step from each tile's
+                                 first slice, so its volume does             */
     JFDK_OPT_FILTER_SIMT = 5, /* 1: ramp product on FP32 CUDA cores (same as
                                  JFDK_OPT_RAMP_PRODUCT = JFDK_RAMP_FP32_SIMT);
                                  0: the form's default                          */
@@ -304,15 +305,15 @@ typedef enum {
     JFDK_RAMP_I8X14 = 5       /* rows and the operator (from its FP64 kernel) as
                                  32-bit fixed point below power-of-two scales, each
                                  cut into four signed bytes; the ten leading byte
-                                 products summed exactly in int32, combined exactly
-                                 in int64, rounded once: the product of the float
+                                 products summed exactly in int32, combined in
+                                 double, rounded once: the product of the float
                                  rows to ~2^-30 of the leading term, independent of
                                  the tiling (the FP32 form's default)            */
 } jfdk_ramp_product;
 jfdk_status jfdk_set_option(jfdk_ctx* ctx, int key, long long value);
 /* The value an option has in effect: the set value, or the default the
- * context resolves it to (JFDK_OPT_BP_ZPT: the tile depth its
- * backprojection runs with; JFDK_OPT_BP_TILE: its tile width;
+ * context resolves it to (JFDK_OPT_BP_ZPT: the depth whose multiples z-slabs
+ * start at, and the tiles' own but for small FP32 launches; JFDK_OPT_BP_TILE: its tile width;
  * JFDK_OPT_RAMP_PRODUCT: the product its filter runs). */
 jfdk_status jfdk_get_option(jfdk_ctx* ctx, int key, long long* value);
 /* Stage times (ms) of the last jfdk_reconstruct with JFDK_OPT_STAGE_TIMING:

@@ -345,8 +345,9 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 4) bp_adjoint_kernel(AdjParams
 // voxels rather than 32 x 1 sample fewer records (L1 hits 84 %); tiles inside
 // the detector run without the range test.  Eight samples in flight at 128
 // registers and 16 warps measured faster than more warps: a 64-view chunk of
-// 256^3 from 512^2 takes 2.1 ms (96 registers and 20 warps 2.9, 80 and 24
-// 3.2; 3.26 with the reduction every 8 samples, 32 x 1 warps and 64 registers).
+// 256^3 from 512^2 takes 2.1 ms, 2.3 with W(z) (96 registers and 20 warps 2.9, 80
+// and 24 3.2; 3.26 with the reduction every 8 samples, 32 x 1 warps and 64
+// registers).
 // J is 1 where 4 would leave less than a full wave of CTAs.
 constexpr int kGradThreads = 128, kGradRows = kGradThreads / 8;   // 8 columns x kGradRows of warps of 4 x 8
 constexpr int kGradRed = 2 * (kGradThreads / 32) * 16;           // floats the CTA's reduction takes, double buffered

@@ -25,12 +25,16 @@ struct BatchTile {
 // parameters sit at a fixed offset of the kernel's parameter space (slot S,
 // a compile-time index), so the tile body reads them as constant operands
 // exactly as the single-scan kernels do; a shared-memory or indexed copy of
-// them measured 16-27 % slower at the 64-register bound.  Each slot holds its
+// them measured 16-27 % slower (at a bound of 64 registers).  Each slot holds its
 // scan's own tile depth (4 or 8 slices, a uniform branch per tile), so scans
 // tuned to either depth share the launch.  DEEP: a launch of the mixed
-// form's 16-slice tiles only, at that body's register bound (96 registers;
-// the 4- and 8-slice bodies run at 64).  The next tile's index is fetched
-// while the current one runs.
+// form's 16-slice tiles only, at that body's register bound (128 registers, four
+// CTAs per SM; the mixed 4- and 8-slice bodies run at 72 and seven, the FP32 ones at
+// 80 and six).  The next tile's index is fetched while the current one runs.
+//
+// Every tile runs the loop with the range test and 64-bit addresses, without the
+// per-scan kernels' sorting of tiles: 16 scans of uneven size 688 GUPS (FP32; the
+// per-scan launches of the pipelined schedule 882) and 986 (mixed; 1252).
 // WV: every scan of the launch divides by its weight volume (p.wvol).
 template <int S, bool MIXED, bool WZ, bool WV, bool DEEP>
 __device__ __forceinline__ void batch_slot_tile(const BatchSlots& t) {

@@ -339,12 +339,15 @@ Geo geometry(const jfdk_ctx* c) {
 }
 
 // Slices per thread: the option, else 16 in the mixed form when W does not
-// depend on z and the volume holds at least 8 waves of 16-slice tiles (5
-// CTAs per SM), 8 otherwise.  16 slices halve the mixed loop's per-view work
-// (87.8 against 93.6 ms on c2, 130 waves), but a small volume then fills the
-// GPU in few waves (c1, 128^3: 1.4 waves, 1.39 against 1.22 ms with 8); the
-// FP32 form measured 139 ms with 16 against 128 with 8 (its per-slice
-// coordinates leave no per-view work to amortise).
+// depend on z and the volume holds at least 40 16-slice tiles per SM, 8 otherwise.
+// 16 slices halve the mixed loop's per-view work, but leave a small volume few
+// tiles: from 360 views of a flexing gantry 128^3 (7 tiles per SM) takes 735 us with
+// 8 and 677 with 16, 160^3 (14) 1233 and 1293, 192^3 (23) 1965 and 1904, 240^3 (49)
+// 3716 and 3587, 320^3 (108) 8372 and 7826; from 40 views 192^3 246 and 259, 256^3
+// (55) 540 and 547, 512 x 512 x 128 (111) 1023 and 993.  (The mixed volume's last
+// bits follow the depth, so the line stays where it is between its two sides.)  The
+// FP32 form measured 139 ms a c2 volume with 16 against 128 with 8: its per-slice
+// coordinates leave no per-view work to amortise.
 int bp_zpt(const jfdk_ctx* c) {
     if (c->opt_bp_zpt) return c->opt_bp_zpt;
     if (!mixed(c) || c->w_depends_on_z) return 8;
@@ -353,8 +356,9 @@ int bp_zpt(const jfdk_ctx* c) {
     return tiles >= 8LL * 5 * c->sms ? 16 : 8;
 }
 
-// The depth a launch over nz slices runs with: in the FP32 form, whose volume
-// does not depend on it, 4 instead of the default 8 where 8-slice tiles fill at
+// The depth a launch over nz slices runs with (jfdk_get_option reports bp_zpt, at
+// whose multiples slabs start): in the FP32 form, whose volume does not depend on it,
+// 4 instead of the default 8 where 8-slice tiles fill at
 // most half of a wave (6 CTAs per SM): 64^3 from 180 views (256 tiles) 280 us
 // against 350; at 864 tiles, nearly a full wave, 708 against 617.
 int launch_zpt(const jfdk_ctx* c, int nz) {
