@@ -624,6 +624,7 @@ void jfdk_destroy(jfdk_ctx* c) {
     dev_free(c, c->d_q4); dev_free(c, c->d_stage); dev_free(c, c->d_qscale); dev_free(c, c->d_absmax);
     dev_free(c, c->d_sum); dev_free(c, c->d_cnt); dev_free(c, c->d_raw_stage); dev_free(c, c->d_hu_stage);
     dev_free(c, c->d_Tt); dev_free(c, c->d_qadj); dev_free(c, c->d_partial);
+    for (float4*& q : c->qadj_kept) dev_free(c, q);
     dev_free(c, c->d_dptm);
     dev_free(c, c->d_wvol);
     for (auto& e : c->ev)
@@ -1294,12 +1295,19 @@ jfdk_status jfdk_bp_adjoint(jfdk_ctx* c, const float* d_vol_bar, int v0, int nv,
     AdjParams a = adj_params(c, d_vol_bar, v0, nv);
     a.qbar = d_q_bar;
     // quad space where it is faster and its scratch is there or can be had (an
-    // allocation would break a capture under way); patches need none
+    // allocation would break a capture under way); patches need none.  Scratch that a
+    // captured graph names stays where it is when a larger call needs more.
+    const bool capture = capturing(c->stream);
     bool quads = !adjoint_by_patches(a, &c->ptms[(size_t)v0 * 12]);
     if (quads && c->qadj_views < nv) {
         quads = false;
-        if (!capturing(c->stream)) {
-            dev_free(c, c->d_qadj);
+        if (!capture) {
+            if (c->qadj_captured)
+                c->qadj_kept.push_back(c->d_qadj);
+            else
+                dev_free(c, c->d_qadj);
+            c->d_qadj = nullptr;
+            c->qadj_captured = false;
             c->qadj_views = 0;
             st = dev_alloc(c, &c->d_qadj, (size_t)nv * frame_px(c), "the quad-space adjoint");
             if (st && st != JFDK_ERR_OOM) return st;
@@ -1307,6 +1315,7 @@ jfdk_status jfdk_bp_adjoint(jfdk_ctx* c, const float* d_vol_bar, int v0, int nv,
         }
     }
     if (quads) {
+        c->qadj_captured |= capture;
         a.quads = c->d_qadj;
         JFDK_LAUNCH(c, launch_bp_adjoint_quads(a, c->w_depends_on_z, c->stream), "backprojection adjoint");
         ++c->launches;   // back to pixels

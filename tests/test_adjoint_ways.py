@@ -82,3 +82,42 @@ def test_rule(name):
     # fewer views of the same scan, from the scratch of more
     sub = _adjoint(scan, vol, vox, tilt, nv=2)[0]
     assert (qb[:2] - sub).double().norm().item() <= 1e-6 * m[:2].double().norm().item()
+
+
+def test_a_captured_call_outlives_larger_ones():
+    """Quad space captured with its scratch in place, then a call of more views: the
+    graph's scratch stays.  Captured before there is any, patches run."""
+    import torch
+
+    from jenhine_b200.fdk import FDKEngine, ReconConfig, ScanConfig
+    from jenhine_b200.phantom import ScanGeometry
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    views, u, v = 12, 60, 50
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        e = FDKEngine(ScanConfig(views, 500.0, 800.0, u, v, 1.0), ReconConfig(20, 20, 16, 1.0, 1.0),
+                      ScanGeometry(views, 500.0, 800.0, u, v, 1.0, 1.0).ptms(), stream=s.cuda_stream)
+        e.bp_reset()
+        e.bp_accumulate(torch.ones((views, v, u), device="cuda"), 0)
+        y = torch.randn((16, 20, 20), device="cuda")
+        outs, graphs = [torch.empty((2, v, u), device="cuda") for _ in range(2)], []
+        held = []
+        for out in outs:
+            torch.cuda.synchronize()
+            graphs.append(torch.cuda.CUDAGraph())
+            with torch.cuda.graph(graphs[-1], stream=s):
+                e.bp_adjoint(y, 0, 2, out=out)
+            torch.cuda.synchronize()
+            held.append(e.device_bytes)
+            want = e.bp_adjoint(y, 0, 2)       # after the first capture: makes the scratch
+        assert held[1] == held[0] + 2 * 16 * u * v
+        whole = e.bp_adjoint(y)
+        for g, out in zip(graphs, outs):
+            out.fill_(np.nan)
+            g.replay()
+            torch.cuda.synchronize()
+            bar = 1e-6 * e.bp_adjoint(y.abs(), 0, 2).double().norm().item()
+            for other in (want, whole[:2]):
+                assert (out - other).double().norm().item() <= bar
+    torch.cuda.synchronize()
