@@ -337,7 +337,10 @@ jfdk_status jfdk_stage_times(jfdk_ctx* ctx, float* ms3);
 jfdk_status jfdk_set_bp_geometry(jfdk_ctx* ctx, const float* h_ptms);
 /* q_bar = S^T (vol_bar / C) for views [v0, v0 + nv): d_vol_bar is
  * num_pixels_z x y x x, d_q_bar nv x rows x filter_out_w.  C is the weight
- * volume of the last jfdk_bp_accumulate sequence (JFDK_ERR_STATE without). */
+ * volume of the last jfdk_bp_accumulate sequence (JFDK_ERR_STATE without).
+ * Scans for which that is faster take 16 bytes of scratch a pixel of the nv
+ * views, kept for later calls; without room for it (or inside a capture that no
+ * call went before) the other way runs, which takes none. */
 jfdk_status jfdk_bp_adjoint(jfdk_ctx* ctx, const float* d_vol_bar, int v0, int nv, float* d_q_bar);
 /* x_bar = w o (T^T y_bar) + (c . y_bar) / 3 on the three edge samples:
  * d_q_bar nv x rows x filter_out_w in, d_p_bar nv x rows x filter_in_w out. */

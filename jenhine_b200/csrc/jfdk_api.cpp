@@ -80,6 +80,30 @@ void dev_free(jfdk_ctx* c, T*& p) {
     p = nullptr;
 }
 
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return true;   // the legacy stream while another stream captures
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// Called by the entry points that use working buffers: from the first call that is
+// captured on, buffers that larger ones replace are kept until the context goes,
+// because the graph names them.
+void note_capture(jfdk_ctx* c) { c->captured = c->captured || capturing(c->stream); }
+
+template <class T>
+void dev_replace(jfdk_ctx* c, T*& p) {
+    if (p && c->captured) {
+        c->kept.push_back(p);
+        p = nullptr;
+    } else {
+        dev_free(c, p);
+    }
+}
+
 // K padded to 64 elements: whole 128-byte rows for every operand kind.
 int a_pitch(const jfdk_ctx* c) { return (int)round_up(c->in_w, 64); }
 long long frame_px(const jfdk_ctx* c) { return (long long)c->rows * c->out_w; }
@@ -106,7 +130,7 @@ size_t a_rows(const jfdk_ctx* c) { return c->a_bytes / a_row_bytes(c); }   // th
 
 jfdk_status ensure_A_bytes(jfdk_ctx* c, size_t bytes) {
     if (c->a_bytes >= bytes) return JFDK_OK;
-    dev_free(c, c->d_A);
+    dev_replace(c, c->d_A);
     c->a_bytes = 0;
     jfdk_status st = dev_alloc(c, reinterpret_cast<char**>(&c->d_A), bytes, "the weighted rows");
     if (!st) c->a_bytes = bytes;
@@ -116,8 +140,8 @@ jfdk_status ensure_A_bytes(jfdk_ctx* c, size_t bytes) {
 jfdk_status ensure_A(jfdk_ctx* c, size_t rows) {
     jfdk_status st = ensure_A_bytes(c, rows * a_row_bytes(c));
     if (st || c->e_rows >= rows) return st;
-    dev_free(c, c->d_e);
-    dev_free(c, c->d_arow);
+    dev_replace(c, c->d_e);
+    dev_replace(c, c->d_arow);
     c->e_rows = 0;
     if ((st = dev_alloc(c, &c->d_e, rows, "the edge means"))) return st;
     if ((st = dev_alloc(c, &c->d_arow, rows, "the row scales"))) return st;
@@ -140,7 +164,7 @@ AOperand a_operand(const jfdk_ctx* c) {
 
 jfdk_status ensure_plain(jfdk_ctx* c, int views) {
     if (c->plain_views >= views) return JFDK_OK;
-    dev_free(c, c->d_plain);
+    dev_replace(c, c->d_plain);
     c->plain_views = 0;
     jfdk_status st = dev_alloc(c, &c->d_plain, (size_t)views * frame_px(c), "the filtered frames");
     if (st) return st;
@@ -154,7 +178,7 @@ size_t record_size(const jfdk_ctx* c) { return mixed(c) ? 8 : 16; }
 
 jfdk_status ensure_Q4(jfdk_ctx* c, int views) {
     if (c->q4_views >= views) return JFDK_OK;
-    dev_free(c, c->d_q4);
+    dev_replace(c, c->d_q4);
     c->q4_views = 0;
     const size_t bytes = (size_t)views * frame_px(c) * record_size(c);
     jfdk_status st = dev_alloc(c, &c->d_q4, (bytes + 15) / 16, "the backprojection store");
@@ -165,7 +189,7 @@ jfdk_status ensure_Q4(jfdk_ctx* c, int views) {
 
 jfdk_status ensure_absmax(jfdk_ctx* c, int n) {
     if (c->absmax_n >= n) return JFDK_OK;
-    dev_free(c, c->d_absmax);
+    dev_replace(c, c->d_absmax);
     c->absmax_n = 0;
     jfdk_status st = dev_alloc(c, &c->d_absmax, (size_t)n, "the per-view maxima");
     if (st) return st;
@@ -394,15 +418,6 @@ jfdk_status pack_frames(jfdk_ctx* c, const float* plain, int nv, int view0, int 
     return JFDK_OK;
 }
 
-bool capturing(cudaStream_t s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
-        cudaGetLastError();
-        return true;   // the legacy stream while another stream captures
-    }
-    return st != cudaStreamCaptureStatusNone;
-}
-
 // The FP32 form's normalisation weights over every view (JFDK_OPT_BP_WEIGHTS),
 // computed once per geometry and rounding mode on the context's stream,
 // which is then synchronised, so later launches on any stream (and graph
@@ -517,6 +532,7 @@ jfdk_status filter_stage_range(jfdk_ctx* c, const uint16_t* d_raw, int vbeg, int
     if (c->in_w != c->used_u && !compositing(c))
         return fail(c, JFDK_ERR_UNSUPPORTED,
                     "reconstruct: filter input width must be the frame width or twice it (compositing)");
+    note_capture(c);
     stage_once(c);
     jfdk_status st = ensure_Q4(c, c->nviews);
     if (st) return st;
@@ -624,7 +640,7 @@ void jfdk_destroy(jfdk_ctx* c) {
     dev_free(c, c->d_q4); dev_free(c, c->d_stage); dev_free(c, c->d_qscale); dev_free(c, c->d_absmax);
     dev_free(c, c->d_sum); dev_free(c, c->d_cnt); dev_free(c, c->d_raw_stage); dev_free(c, c->d_hu_stage);
     dev_free(c, c->d_Tt); dev_free(c, c->d_qadj); dev_free(c, c->d_partial);
-    for (float4*& q : c->qadj_kept) dev_free(c, q);
+    for (void*& q : c->kept) dev_free(c, q);
     dev_free(c, c->d_dptm);
     dev_free(c, c->d_wvol);
     for (auto& e : c->ev)
@@ -947,6 +963,7 @@ jfdk_status jfdk_preprocess_frames(jfdk_ctx* c, const uint16_t* d_raw, int nv, f
 jfdk_status jfdk_filter_frames(jfdk_ctx* c, const float* d_in, int v0, int nv, float* d_out) {
     if (!c || !d_in || !d_out || nv < 0 || v0 < 0) return fail(c, JFDK_ERR_INVALID, "filter: bad argument");
     if (nv == 0) return JFDK_OK;
+    note_capture(c);
     jfdk_status st = ensure_A(c, (size_t)nv * c->rows);
     if (st) return st;
     JFDK_LAUNCH(c, launch_weight(d_in, nv, v0, c->in_w, c->rows, weight_params(c), a_operand(c), c->d_e, c->stream),
@@ -1007,6 +1024,7 @@ jfdk_status jfdk_bp_accumulate(jfdk_ctx* c, const float* d_proj, int v0, int nv)
         return fail(c, JFDK_ERR_INVALID, "bp_accumulate: bad argument");
     if (!c->d_sum) return fail(c, JFDK_ERR_STATE, "bp_accumulate before bp_reset");
     if (nv == 0) return JFDK_OK;
+    note_capture(c);
     jfdk_status st = ensure_Q4(c, nv);
     if (st) return st;
     // InitView: taper the caller's frames while packing them
@@ -1061,6 +1079,7 @@ jfdk_status jfdk_filter_raw(jfdk_ctx* c, const uint16_t* d_raw, int v0, int nv, 
         return fail(c, JFDK_ERR_UNSUPPORTED,
                     "filter_raw: filter input width must be the frame width or twice it (compositing)");
     int chunk = 0;
+    note_capture(c);
     jfdk_status st = ensure_chunk(c, false, &chunk);
     if (st) return st;
     const size_t frame = (size_t)c->scan.num_dets_u * c->scan.num_dets_v;
@@ -1295,19 +1314,13 @@ jfdk_status jfdk_bp_adjoint(jfdk_ctx* c, const float* d_vol_bar, int v0, int nv,
     AdjParams a = adj_params(c, d_vol_bar, v0, nv);
     a.qbar = d_q_bar;
     // quad space where it is faster and its scratch is there or can be had (an
-    // allocation would break a capture under way); patches need none.  Scratch that a
-    // captured graph names stays where it is when a larger call needs more.
-    const bool capture = capturing(c->stream);
+    // allocation would break a capture under way); patches need none
+    note_capture(c);
     bool quads = !adjoint_by_patches(a, &c->ptms[(size_t)v0 * 12]);
     if (quads && c->qadj_views < nv) {
         quads = false;
-        if (!capture) {
-            if (c->qadj_captured)
-                c->qadj_kept.push_back(c->d_qadj);
-            else
-                dev_free(c, c->d_qadj);
-            c->d_qadj = nullptr;
-            c->qadj_captured = false;
+        if (!capturing(c->stream)) {
+            dev_replace(c, c->d_qadj);
             c->qadj_views = 0;
             st = dev_alloc(c, &c->d_qadj, (size_t)nv * frame_px(c), "the quad-space adjoint");
             if (st && st != JFDK_ERR_OOM) return st;
@@ -1315,7 +1328,6 @@ jfdk_status jfdk_bp_adjoint(jfdk_ctx* c, const float* d_vol_bar, int v0, int nv,
         }
     }
     if (quads) {
-        c->qadj_captured |= capture;
         a.quads = c->d_qadj;
         JFDK_LAUNCH(c, launch_bp_adjoint_quads(a, c->w_depends_on_z, c->stream), "backprojection adjoint");
         ++c->launches;   // back to pixels
@@ -1331,6 +1343,7 @@ jfdk_status jfdk_filter_adjoint(jfdk_ctx* c, const float* d_q_bar, int v0, int n
     const int kp = (int)round_up(c->out_w, 64);
     const size_t m = (size_t)nv * c->rows;
     // the padded rows of q_bar go where the forward keeps its A operand
+    note_capture(c);
     jfdk_status st = ensure_A_bytes(c, m * kp * sizeof(float));
     if (st) return st;
     float* ypad = static_cast<float*>(c->d_A);
@@ -1354,6 +1367,7 @@ jfdk_status jfdk_geometry_gradient(jfdk_ctx* c, const float* d_q, int v0, int nv
         return fail(c, JFDK_ERR_INVALID, "geometry_gradient: bad argument");
     jfdk_status st = deriv_check(c, "geometry_gradient");
     if (st || nv == 0) return st;
+    note_capture(c);
     if ((st = ensure_Q4(c, nv))) return st;
     JFDK_LAUNCH(c, launch_pack_quads(d_q, frame_px(c), nv, c->rows, c->out_w, c->d_tw, v0, c->nviews, 1, c->d_q4,
                                      frame_px(c), 0, c->stream),
@@ -1364,7 +1378,7 @@ jfdk_status jfdk_geometry_gradient(jfdk_ctx* c, const float* d_q, int v0, int nv
     a.dptm = d_dptm;
     const size_t need = geometry_gradient_ctas(a) * 6 * (size_t)nv;
     if (c->partial_n < need) {
-        dev_free(c, c->d_partial);
+        dev_replace(c, c->d_partial);
         c->partial_n = 0;
         if ((st = dev_alloc(c, &c->d_partial, need, "the gradient partial sums"))) return st;
         c->partial_n = need;

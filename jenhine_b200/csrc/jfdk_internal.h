@@ -353,8 +353,9 @@ struct jfdk_ctx {
     bool bp_has_views = false;
     // derivatives (allocated on demand)
     float4* d_qadj = nullptr; int qadj_views = 0;    // quad-space adjoint
-    bool qadj_captured = false;                      // a captured graph names d_qadj
-    std::vector<float4*> qadj_kept;                  // former ones that graphs name, freed with the context
+    // a call was captured: from then on working buffers that larger ones replace are kept
+    bool captured = false;
+    std::vector<void*> kept;
     float* d_partial = nullptr; size_t partial_n = 0;
     float* d_dptm = nullptr; int dptm_views = 0;
 

@@ -97,3 +97,39 @@ def test_another_product_in_the_same_buffers():
     for product in (*want, *reversed(want)):
         e.set_option(_lib.OPT_RAMP_PRODUCT, product)
         assert torch.equal(e.reconstruct(raw).nan_to_num(1e30), want[product].nan_to_num(1e30)), product
+
+
+@pytest.mark.parametrize("later", ["more_views", "another_product", "adjoint"])
+def test_buffers_a_graph_names_are_kept(later):
+    """A captured filter call, then one that needs larger buffers: more views, rows of
+    two TF32 parts, the filter adjoint of many views."""
+    import torch
+
+    from jenhine_b200 import _lib
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        e, _, raw = _engine(stream=s.cuda_stream)
+        frames = e.preprocess(raw)
+        want = e.filter(frames[:2])
+        out = torch.empty_like(want)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            e.filter(frames[:2], out=out)
+        torch.cuda.synchronize()
+        held = e.device_bytes
+        if later == "more_views":
+            e.filter(frames)
+        elif later == "another_product":
+            e.set_option(_lib.OPT_RAMP_PRODUCT, _lib.RAMP_TF32X3)
+            e.filter(frames[:2])
+        else:
+            e.filter_adjoint(frames)
+        assert e.device_bytes > held
+        junk = torch.full((1 << 22,), np.nan, device="cuda")
+        out.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) and junk.isnan().all()
